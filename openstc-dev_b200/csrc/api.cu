@@ -669,6 +669,23 @@ void build_devparam(const ostc_param *p, DevParam &d) {
     }
     d.t_low[i] = p->t_low[i];
     d.t_mid[i] = p->t_mid[i];
+    {
+      // below t_low: cp = cp(t_low), h = h(t_low) + cp(t_low) (t - t_low), a constant and a
+      // linear term; nz_ext is its difference from the low range
+      const double *c = d.lo[i], tl = p->t_low[i];
+      const double cp = c[0] + tl * (c[1] + tl * (c[2] + tl * (c[3] + tl * c[4])));
+      const double h = c[5] + tl * (c[0] + tl * (c[1] / 2 + tl * (c[2] / 3 + tl * (c[3] / 4 + tl * c[4] / 5))));
+      const double ext[6] = {cp, 0, 0, 0, 0, h - cp * tl};
+      for (int k = 0; k < 6; ++k) {
+        d.nz_lo[i][k] = d.lo[i][k] * d.Rmw[i];
+        d.nz_hi[i][k] = d.hi[i][k] * d.Rmw[i];
+        d.nz_ext[i][k] = (ext[k] - d.lo[i][k]) * d.Rmw[i];
+      }
+    }
+    const double up = std::max(d.t_mid[i], d.t_low[i]);  // the high range starts here
+    d.tmid_min = i ? std::min(d.tmid_min, up) : up;
+    d.tmid_max = i ? std::max(d.tmid_max, up) : up;
+    d.tlow_max = i ? std::max(d.tlow_max, d.t_low[i]) : d.t_low[i];
     d.LJ_inv[i] = p->LJ_potent_inv[i];
     d.vis_coeff[i] = p->vis_coeff[i];
     d.LJm145[i] = std::pow(p->LJ_potent_inv[i], -0.145);

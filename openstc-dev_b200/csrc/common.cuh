@@ -43,6 +43,12 @@ struct DevParam {
   double A[MAXR], b[MAXR], Ea[MAXR], A2[MAXR], b2[MAXR], Ea2[MAXR];
   double tb[MAXR][MAXS];                           // third-body efficiencies
   double troe_alpha[MAXR], troe_t3[MAXR], troe_t1[MAXR], troe_t2[MAXR];
+  // the ranges times R_u/W_k for sums over the species (nasa_sums, thermo.cuh):
+  // c[0..5] of the low and high ranges, and what the linear extension below
+  // t_low adds to the low range; the lowest and highest start of a
+  // high range (t_mid, or t_low above it) and the highest t_low
+  double nz_lo[MAXS][6], nz_hi[MAXS][6], nz_ext[MAXS][6];
+  double tmid_min, tmid_max, tlow_max;
 };
 
 // c_p (the __constant__ DevParam) is defined in kernels.cu before the

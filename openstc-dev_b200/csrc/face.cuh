@@ -100,34 +100,38 @@ struct TileCells {
 };
 
 // 0.5 * (sgn(a) + sgn(b)) * min(|a|, |b|) with sgn(x) = (x < 0 ? -1 : 1)
-// (Limiter.cuh:13-16), written without the integer sum and its conversion:
-// the product is exactly +m, -m or +0, so the result is bit-identical;
-// symmetric in a and b
+// (Limiter.cuh:13-16): the one of smaller magnitude, or 0 where the signs
+// differ. Signs by comparison, so that a NaN counts as positive; where one
+// argument is NaN the magnitude is the other's, as fmin's. Symmetric in a and
+// b up to the sign of a zero.
 __device__ __forceinline__ double minmod(double a, double b) {
-  const double m = fmin(fabs(a), fabs(b));
-  const bool na = a < 0, nb = b < 0;
-  return na != nb ? 0.0 : (na ? -m : m);
+  const bool b_nan = (__double2hiint(b) & 0x7fffffff) >= 0x7ff00000;  // (or infinite: then a is no larger)
+  const double m = (fabs(a) < fabs(b) || b_nan) ? a : b;
+  return (a < 0) != (b < 0) ? 0.0 : m;
 }
 
 // ---------------------------------------------------------------------------
 // Riemann solvers on reconstructed states (pl/pr: NV primitive values, then
-// total energy at NV and gamma at NV+1). Output: NV face fluxes.
+// total energy at NV, gamma at NV+1, total enthalpy (E + p) / rho at NV+2 and
+// p / rho at NV+3). Output: NV face fluxes. Quotients by the same divisor are
+// products with one reciprocal: an FP64 division is a sequence of about twenty
+// instructions, and these faces are bound by the instructions they issue.
 // ---------------------------------------------------------------------------
 // AUSM+ (AusmP.cu:6-94); k1..k3: jac-weighted face metric
 template <int NV, bool MIXG>
 __device__ __forceinline__ void ausm_plus(const double *pl, const double *pr, double k1, double k2, double k3,
                                           double *F) {
   const double gk = sqrt(k1 * k1 + k2 * k2 + k3 * k3);
-  const double ul = (k1 * pl[1] + k2 * pl[2] + k3 * pl[3]) / gk;
-  const double ur = (k1 * pr[1] + k2 * pr[2] + k3 * pr[3]) / gk;
   const double gl = MIXG ? pl[NV + 1] : gamma_air, gr = MIXG ? pr[NV + 1] : gamma_air;
-  const double c = 0.5 * (sqrt(gl * pl[4] / pl[0]) + sqrt(gr * pr[4] / pr[0]));
-  const double mlm = ul / c, mrm = ur / c;
+  const double c = 0.5 * (sqrt(gl * pl[NV + 3]) + sqrt(gr * pr[NV + 3]));
+  const double igc = 1.0 / (gk * c);
+  const double mlm = (k1 * pl[1] + k2 * pl[2] + k3 * pl[3]) * igc;
+  const double mrm = (k1 * pr[1] + k2 * pr[2] + k3 * pr[3]) * igc;
   double mlp, mrn, plp, prn;
   constexpr double alpha = 3 / 16.0;
   if (fabs(mlm) > 1) {
     mlp = 0.5 * (mlm + fabs(mlm));
-    plp = mlp / mlm;
+    plp = mlm > 0 ? 1.0 : 0.0;  // mlp / mlm
   } else {
     const double a = (mlm + 1) * (mlm + 1) * 0.25;
     const double b = (mlm * mlm - 1) * (mlm * mlm - 1);
@@ -136,7 +140,7 @@ __device__ __forceinline__ void ausm_plus(const double *pl, const double *pr, do
   }
   if (fabs(mrm) > 1) {
     mrn = 0.5 * (mrm - fabs(mrm));
-    prn = mrn / mrm;
+    prn = mrm < 0 ? 1.0 : 0.0;  // mrn / mrm
   } else {
     const double a = (mrm - 1) * (mrm - 1) * 0.25;
     const double b = (mrm * mrm - 1) * (mrm * mrm - 1);
@@ -148,13 +152,12 @@ __device__ __forceinline__ void ausm_plus(const double *pl, const double *pr, do
   const double mass = c * (pl[0] * 0.5 * (mh + fabs(mh)) + pr[0] * 0.5 * (mh - fabs(mh)));
   const double co = mass * gk;
   const bool left = mass >= 0;
-  const double q0 = left ? pl[0] : pr[0], q1 = left ? pl[1] : pr[1], q2 = left ? pl[2] : pr[2];
-  const double q3 = left ? pl[3] : pr[3], q4 = left ? pl[4] : pr[4], qe = left ? pl[NV] : pr[NV];
+  const double q1 = left ? pl[1] : pr[1], q2 = left ? pl[2] : pr[2], q3 = left ? pl[3] : pr[3];
   F[0] = co;
   F[1] = co * q1 + pc * k1;
   F[2] = co * q2 + pc * k2;
   F[3] = co * q3 + pc * k3;
-  F[4] = co * (qe + q4) / q0;
+  F[4] = co * (left ? pl[NV + 2] : pr[NV + 2]);
 #pragma unroll
   for (int l = 5; l < NV; ++l) F[l] = co * (left ? pl[l] : pr[l]);
 }
@@ -163,13 +166,12 @@ __device__ __forceinline__ void ausm_plus(const double *pl, const double *pr, do
 template <int NV, int NS>
 __device__ __forceinline__ void hllc(const double *pl, const double *pr, double kx, double ky, double kz,
                                      double jac_ave, double *F) {
-  const double sl0 = sqrt(pl[0]), sr0 = sqrt(pr[0]);
-  const double rlc = sl0 / (sl0 + sr0), rrc = sr0 / (sl0 + sr0);
+  const double sl0 = sqrt(pl[0]), sr0 = sqrt(pr[0]), isum = 1.0 / (sl0 + sr0);
+  const double rlc = sl0 * isum, rrc = sr0 * isum;
   const double ut = pl[1] * rlc + pr[1] * rrc;
   const double vt = pl[2] * rlc + pr[2] * rrc;
   const double wt = pl[3] * rlc + pr[3] * rrc;
-  const double hl = (pl[NV] + pl[4]) / pl[0], hr = (pr[NV] + pr[4]) / pr[0];
-  const double ht = hl * rlc + hr * rrc;
+  const double ht = pl[NV + 2] * rlc + pr[NV + 2] * rrc;
   const double ekt = 0.5 * (ut * ut + vt * vt + wt * wt);
   double c_tilde;
   if constexpr (NS == 0) {
@@ -181,26 +183,24 @@ __device__ __forceinline__ void hllc(const double *pl, const double *pr, double 
       svm[l] = rlc * pl[l + 5] + rrc * pr[l + 5];
       mw_inv += svm[l] * c_p.imw[l];
     }
-    const double t = (rlc * (pl[4] / pl[0]) + rrc * (pr[4] / pr[0])) / (R_u * mw_inv);
-    double h_i[NS], cp_i[NS];
-    enthalpy_cp<NS>(t, h_i, cp_i);
-    double cvv = 0, cpp = 0;
-#pragma unroll
-    for (int l = 0; l < NS; ++l) {
-      cpp += cp_i[l] * svm[l];
-      cvv += svm[l] * (cp_i[l] - c_p.Rmw[l]);
-    }
-    c_tilde = sqrt(cpp / cvv * R_u * mw_inv * t);
+    const double R = R_u * mw_inv, rt = rlc * pl[NV + 3] + rrc * pr[NV + 3];  // R T of the mean state
+    const double t = rt / R;
+    double A[6];
+    nasa_sums<NS>(t, [&](int l) { return svm[l]; }, A);
+    const double cp = nasa_cp(A, t);
+    c_tilde = sqrt(cp / (cp - R) * rt);
   }
-  const double gradK = sqrt(kx * kx + ky * ky + kz * kz);
-  const double Ub = (kx * ut + ky * vt + kz * wt) / gradK;
+  const double gradK = sqrt(kx * kx + ky * ky + kz * kz), igk = 1.0 / gradK;
+  const double Ub = (kx * ut + ky * vt + kz * wt) * igk;
   const double gl = NS > 0 ? pl[NV + 1] : gamma_air, gr = NS > 0 ? pr[NV + 1] : gamma_air;
   const double Ul = kx * pl[1] + ky * pl[2] + kz * pl[3];
-  const double cl = sqrt(gl * pl[4] / pl[0]);
-  const double sl = fmin(Ul / gradK - cl, Ub - c_tilde);
+  const double cl = sqrt(gl * pl[NV + 3]);
+  const double uln = Ul * igk;  // velocities along the unit normal
+  const double sl = fmin(uln - cl, Ub - c_tilde);
   const double Ur = kx * pr[1] + ky * pr[2] + kz * pr[3];
-  const double cr = sqrt(gr * pr[4] / pr[0]);
-  const double sr = fmax(Ur / gradK + cr, Ub + c_tilde);
+  const double cr = sqrt(gr * pr[NV + 3]);
+  const double urn = Ur * igk;
+  const double sr = fmax(urn + cr, Ub + c_tilde);
   if (sl >= 0 || sr < 0) {
     const double *q = sl >= 0 ? pl : pr;
     const double U = sl >= 0 ? Ul : Ur;
@@ -214,9 +214,9 @@ __device__ __forceinline__ void hllc(const double *pl, const double *pr, double 
     for (int l = 5; l < NV; ++l) F[l] = jac_ave * rhoUk * q[l];
     return;
   }
-  const double sm = ((pr[0] * Ur * (sr - Ur / gradK) - pl[0] * Ul * (sl - Ul / gradK)) / gradK + pl[4] - pr[4]) /
-                    (pr[0] * (sr - Ur / gradK) - pl[0] * (sl - Ul / gradK));
-  const double pm = pl[0] * (sl - Ul / gradK) * (sm - Ul / gradK) + pl[4];
+  const double ml = pl[0] * (sl - uln), mr = pr[0] * (sr - urn);
+  const double sm = (urn * mr - uln * ml + pl[4] - pr[4]) / (mr - ml);
+  const double pm = ml * (sm - uln) + pl[4];
   const bool lft = sm >= 0;
   const double *q = lft ? pl : pr;
   const double s = lft ? sl : sr, U = lft ? Ul : Ur;
@@ -227,7 +227,8 @@ __device__ __forceinline__ void hllc(const double *pl, const double *pr, double 
   F[1] = Q * q[1] + dP * kx;
   F[2] = Q * q[2] + dP * ky;
   F[3] = Q * q[3] + dP * kz;
-  F[4] = Q * q[NV] / q[0] + pC * jac_ave * (s * pm * sm * gradK - sm * q[4] * U);
+  // E / rho = (E + p) / rho - p / rho
+  F[4] = Q * (q[NV + 2] - q[NV + 3]) + pC * jac_ave * (s * pm * sm * gradK - sm * q[4] * U);
 #pragma unroll
   for (int l = 5; l < NV; ++l) F[l] = Q * q[l];
 }
@@ -271,6 +272,31 @@ __device__ __forceinline__ void riemann(const double *pl, const double *pr, cons
 // primitive-variable reconstruction face (InviscidScheme.cu:48-158 +
 // Reconstruction.cu:5-46 + Reconstruction.cuh:20-72)
 // ---------------------------------------------------------------------------
+// total energy, gamma, total enthalpy and p / rho of a reconstructed state
+// (entries NV .. NV+3) from its NV primitive values
+template <int NV, int NS>
+__device__ __forceinline__ void face_energy(double *q) {
+  const double ek = 0.5 * (q[1] * q[1] + q[2] * q[2] + q[3] * q[3]);
+  const double pr = q[4] / q[0];
+  q[NV + 3] = pr;
+  if constexpr (NS > 0) {
+    double mw = 0;
+#pragma unroll
+    for (int l = 0; l < NS; ++l) mw += q[5 + l] * c_p.imw[l];
+    const double R = R_u * mw, t = pr / R;
+    double A[6];
+    nasa_sums<NS>(t, [&](int l) { return q[5 + l]; }, A);
+    const double cp = nasa_cp(A, t);
+    q[NV + 2] = ek + nasa_h(A, t);
+    q[NV] = q[0] * q[NV + 2] - q[4];
+    q[NV + 1] = cp / (cp - R);
+  } else {
+    q[NV] = ek * q[0] + q[4] / (gamma_air - 1);
+    q[NV + 1] = gamma_air;
+    q[NV + 2] = ek + pr * (gamma_air / (gamma_air - 1));
+  }
+}
+
 // NT: turbulence scalars (k, omega) after the NS species, reconstructed alike
 template <int NS, int NT, class Cells>
 __device__ __forceinline__ void reconstruct_pv_c(const Cells &c, double *pl, double *pr) {
@@ -298,47 +324,8 @@ __device__ __forceinline__ void reconstruct_pv_c(const Cells &c, double *pl, dou
       pr[l] = v1;
     }
   }
-  if constexpr (NS > 0) {
-    double el = 0.5 * (pl[1] * pl[1] + pl[2] * pl[2] + pl[3] * pl[3]);
-    double er = 0.5 * (pr[1] * pr[1] + pr[2] * pr[2] + pr[3] * pr[3]);
-    double mwl = 0, mwr = 0;
-#pragma unroll
-    for (int l = 0; l < NS; ++l) {
-      mwl += pl[5 + l] * c_p.imw[l];
-      mwr += pr[5 + l] * c_p.imw[l];
-    }
-    const double tl = pl[4] / (pl[0] * R_u * mwl), tr = pr[4] / (pr[0] * R_u * mwr);
-    double cpl = 0, cpr = 0, cvl = 0, cvr = 0;
-    {
-      double h[NS], cp[NS];
-      enthalpy_cp<NS>(tl, h, cp);
-#pragma unroll
-      for (int l = 0; l < NS; ++l) {
-        cpl += cp[l] * pl[l + 5];
-        cvl += pl[l + 5] * (cp[l] - c_p.Rmw[l]);
-        el += h[l] * pl[l + 5];
-      }
-    }
-    {
-      double h[NS], cp[NS];
-      enthalpy_cp<NS>(tr, h, cp);
-#pragma unroll
-      for (int l = 0; l < NS; ++l) {
-        cpr += cp[l] * pr[l + 5];
-        cvr += pr[l + 5] * (cp[l] - c_p.Rmw[l]);
-        er += h[l] * pr[l + 5];
-      }
-    }
-    pl[NV] = pl[0] * el - pl[4];
-    pr[NV] = pr[0] * er - pr[4];
-    pl[NV + 1] = cpl / cvl;
-    pr[NV + 1] = cpr / cvr;
-  } else {
-    pl[NV] = 0.5 * (pl[1] * pl[1] + pl[2] * pl[2] + pl[3] * pl[3]) * pl[0] + pl[4] / (gamma_air - 1);
-    pr[NV] = 0.5 * (pr[1] * pr[1] + pr[2] * pr[2] + pr[3] * pr[3]) * pr[0] + pr[4] / (gamma_air - 1);
-    pl[NV + 1] = gamma_air;
-    pr[NV + 1] = gamma_air;
-  }
+  face_energy<NV, NS>(pl);
+  face_energy<NV, NS>(pr);
 }
 
 template <int NS, int DIR, int NT = 0>
@@ -349,7 +336,7 @@ __device__ __forceinline__ void reconstruct_pv(const DevZone &z, int g0, double 
 template <int NS, int DIR, int NT, class Cells>
 __device__ __forceinline__ void inviscid_face_pv(const Cells &c, double *F) {
   constexpr int NV = 5 + NS + NT;
-  double pl[NV + 2], pr[NV + 2];
+  double pl[NV + 4], pr[NV + 4];
   reconstruct_pv_c<NS, NT>(c, pl, pr);
   riemann<NV, NS>(pl, pr, c, DIR, F);
 }
@@ -378,7 +365,7 @@ template <int NS, int DIR>
 __device__ __forceinline__ void inviscid_face_roe(const DevZone &z, int g0, double *F) {
   constexpr int NV = 5 + NS;
   const int g1 = g0 + dir_stride<DIR>(z);
-  double pl[NV + 2], pr[NV + 2];
+  double pl[NV + 4], pr[NV + 4];
   reconstruct_pv<NS, DIR>(z, g0, pl, pr);
   const double j0 = ld(z.jac + g0), j1 = ld(z.jac + g1);
   const double m0x = met(z, g0, 3 * DIR), m0y = met(z, g0, 3 * DIR + 1), m0z = met(z, g0, 3 * DIR + 2);
@@ -636,21 +623,27 @@ __device__ __forceinline__ void inviscid_face_aweno(const DevZone &z, int g0, do
       }
     }
   }
-  double pl[NV + 2], pr[NV + 2];
+  double pl[NV + 4], pr[NV + 4];
+  const double il = 1.0 / ql[0];
   pl[0] = ql[0];
-  pl[1] = ql[1] / ql[0];
-  pl[2] = ql[2] / ql[0];
-  pl[3] = ql[3] / ql[0];
+  pl[1] = ql[1] * il;
+  pl[2] = ql[2] * il;
+  pl[3] = ql[3] * il;
   pl[4] = gm1 * (ql[4] - 0.5 * (pl[1] * pl[1] + pl[2] * pl[2] + pl[3] * pl[3]) * ql[0]);
   pl[NV] = ql[4];
   pl[NV + 1] = gamma_air;
+  pl[NV + 2] = (ql[4] + pl[4]) * il;
+  pl[NV + 3] = pl[4] * il;
+  const double ir = 1.0 / qr[0];
   pr[0] = qr[0];
-  pr[1] = qr[1] / qr[0];
-  pr[2] = qr[2] / qr[0];
-  pr[3] = qr[3] / qr[0];
+  pr[1] = qr[1] * ir;
+  pr[2] = qr[2] * ir;
+  pr[3] = qr[3] * ir;
   pr[4] = gm1 * (qr[4] - 0.5 * (pr[1] * pr[1] + pr[2] * pr[2] + pr[3] * pr[3]) * qr[0]);
   pr[NV] = qr[4];
   pr[NV + 1] = gamma_air;
+  pr[NV + 2] = (qr[4] + pr[4]) * ir;
+  pr[NV + 3] = pr[4] * ir;
 #pragma unroll
   for (int t = 0; t < NT; ++t) {  // componentwise WENO5 of rho k, rho omega
     double v[6];
@@ -658,8 +651,8 @@ __device__ __forceinline__ void inviscid_face_aweno(const DevZone &z, int g0, do
     for (int s = 0; s < 6; ++s) v[s] = cvl(z, g0 + (s - 2) * sd, 5 + t);
     double vmn = 0, vpl = 0;
     if (c_p.reconstruction == 4) weno5_pair(v, vmn, vpl);
-    pl[5 + t] = vmn / ql[0];
-    pr[5 + t] = vpl / qr[0];
+    pl[5 + t] = vmn * il;
+    pr[5 + t] = vpl * ir;
   }
   riemann<NV, 0>(pl, pr, plane_cells<DIR>(z, g0), DIR, F);
 }
@@ -717,11 +710,17 @@ __device__ __forceinline__ void viscous_face(const Cells &cc, double *F) {
   double mm[9];
 #pragma unroll
   for (int c = 0; c < 9; ++c) mm[c] = 0.5 * (cc.met(c, 0) + cc.met(c, 1));
+  // four times the tangential derivatives are taken: their quarter goes into the metric
+#pragma unroll
+  for (int c = 0; c < 3; ++c) {
+    mm[3 * TA + c] *= 0.25;
+    mm[3 * TB + c] *= 0.25;
+  }
   // derivative along (normal, ta, tb) ordered as (xi, eta, zeta); v(n, a, b) is the variable's cell value
   auto der = [&](auto v, double out[3]) {
     const double dn = v(1, 0, 0) - v(0, 0, 0);
-    const double da = 0.25 * (v(0, 1, 0) - v(0, -1, 0) + v(1, 1, 0) - v(1, -1, 0));
-    const double db = 0.25 * (v(0, 0, 1) - v(0, 0, -1) + v(1, 0, 1) - v(1, 0, -1));
+    const double da = v(0, 1, 0) - v(0, -1, 0) + v(1, 1, 0) - v(1, -1, 0);
+    const double db = v(0, 0, 1) - v(0, 0, -1) + v(1, 0, 1) - v(1, 0, -1);
     out[DIR] = dn;
     out[TA] = da;
     out[TB] = db;
@@ -762,6 +761,10 @@ __device__ __forceinline__ void viscous_face(const Cells &cc, double *F) {
   const double kxj = 0.5 * (cc.met(3 * DIR, 0) * j0 + cc.met(3 * DIR, 1) * j1);
   const double kyj = 0.5 * (cc.met(3 * DIR + 1, 0) * j0 + cc.met(3 * DIR + 1, 1) * j1);
   const double kzj = 0.5 * (cc.met(3 * DIR + 2, 0) * j0 + cc.met(3 * DIR + 2, 1) * j1);
+  // the face-normal gradient of a scalar is one product with its derivatives
+  double kd[3];
+#pragma unroll
+  for (int d = 0; d < 3; ++d) kd[d] = kxj * mm[3 * d] + kyj * mm[3 * d + 1] + kzj * mm[3 * d + 2];
   F[0] = 0;
   F[1] = kxj * txx + kyj * txy + kzj * txz;
   F[2] = kxj * txy + kyj * tyy + kzj * tyz;
@@ -769,12 +772,9 @@ __device__ __forceinline__ void viscous_face(const Cells &cc, double *F) {
   const double um = 0.5 * (cc.bv(1, 0) + cc.bv(1, 1));
   const double vm = 0.5 * (cc.bv(2, 0) + cc.bv(2, 1));
   const double wm = 0.5 * (cc.bv(3, 0) + cc.bv(3, 1));
-  const double t_x = dt[0] * mm[0] + dt[1] * mm[3] + dt[2] * mm[6];
-  const double t_y = dt[0] * mm[1] + dt[1] * mm[4] + dt[2] * mm[7];
-  const double t_z = dt[0] * mm[2] + dt[1] * mm[5] + dt[2] * mm[8];
   double cond = 0.5 * (cc.kappa(0) + cc.kappa(1));
   if constexpr (NT > 0) cond += 0.5 * (cc.ttc(0) + cc.ttc(1));
-  F[4] = um * F[1] + vm * F[2] + wm * F[3] + cond * (kxj * t_x + kyj * t_y + kzj * t_z);
+  F[4] = um * F[1] + vm * F[2] + wm * F[3] + cond * (kd[0] * dt[0] + kd[1] * dt[1] + kd[2] * dt[2]);
   if constexpr (NS > 0) {
     double yk[NS], diff[NS], ddf[NS];
     double sgw = 0, srdy = 0, corr = 0, mwt = 0;
@@ -785,10 +785,7 @@ __device__ __forceinline__ void viscous_face(const Cells &cc, double *F) {
       if constexpr (NT > 0) diff[l] += mut / c_p.Sct;  // turbulent diffusivity (ViscousScheme.cuh:122-125)
       double dy[3];
       der(svv(l), dy);
-      const double y_x = dy[0] * mm[0] + dy[1] * mm[3] + dy[2] * mm[6];
-      const double y_y = dy[0] * mm[1] + dy[1] * mm[4] + dy[2] * mm[7];
-      const double y_z = dy[0] * mm[2] + dy[1] * mm[5] + dy[2] * mm[8];
-      const double g = kxj * y_x + kyj * y_y + kzj * y_z;
+      const double g = kd[0] * dy[0] + kd[1] * dy[1] + kd[2] * dy[2];
       ddf[l] = g;
       corr += diff[l] * g;
       sgw += g * c_p.imw[l];
@@ -800,24 +797,20 @@ __device__ __forceinline__ void viscous_face(const Cells &cc, double *F) {
     if (c_p.gradP) {
       double dp[3];
       der(bvv(4), dp);
-      const double p_x = dp[0] * mm[0] + dp[1] * mm[3] + dp[2] * mm[6];
-      const double p_y = dp[0] * mm[1] + dp[1] * mm[4] + dp[2] * mm[7];
-      const double p_z = dp[0] * mm[2] + dp[1] * mm[5] + dp[2] * mm[8];
-      const double gp = (kxj * p_x + kyj * p_y + kzj * p_z) / (0.5 * (cc.bv(4, 1) + cc.bv(4, 0)));
+      const double gp = (kd[0] * dp[0] + kd[1] * dp[1] + kd[2] * dp[2]) / (0.5 * (cc.bv(4, 1) + cc.bv(4, 0)));
 #pragma unroll
       for (int l = 0; l < NS; ++l) {
         ddf[l] += (mwt * c_p.imw[l] - 1) * yk[l] * gp;
         corr += (mwt * c_p.imw[l] - 1) * yk[l] * gp * diff[l];
       }
     }
-    double h[NS];
-    enthalpy<NS>(0.5 * (cc.bv(5, 0) + cc.bv(5, 1)), h);
+    const double msg = mwt * sgw;
 #pragma unroll
-    for (int l = 0; l < NS; ++l) {
-      const double flux = diff[l] * (ddf[l] - mwt * yk[l] * sgw) - yk[l] * corr;
-      F[5 + l] = flux;
-      F[4] += h[l] * flux;
-    }
+    for (int l = 0; l < NS; ++l) F[5 + l] = diff[l] * (ddf[l] - msg * yk[l]) - yk[l] * corr;
+    const double tm = 0.5 * (cc.bv(5, 0) + cc.bv(5, 1));
+    double A[6];
+    nasa_sums<NS>(tm, [&](int l) { return F[5 + l]; }, A);
+    F[4] += nasa_h(A, tm);  // sum of h_l times the diffusive fluxes
   }
   if constexpr (NT > 0) {  // k and omega diffusion (ViscousScheme.cuh:200-251)
     double dk[3], dw[3];
