@@ -488,34 +488,28 @@ __device__ __forceinline__ void inviscid_face_roe(const DevZone &z, int g0, doub
 // rows are processed one at a time so that only one row of the left
 // eigenvector matrix is live.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void weno5_pair(const double v[6], double &vminus, double &vplus) {
+// WENO5 value at one side of the face from the five cells w0..w4 in the order
+// away from it (AWENO.cu: the other side takes them reversed). The weights
+// d_i (1 + tau / (eps + b_i)^2) are taken times the product of the three
+// (eps + b_i)^2, which cancels in the quotient: one division where the weights
+// one by one take four. The product stays in range for characteristic values
+// below 1e25.
+__device__ __forceinline__ double weno5(double w0, double w1, double w2, double w3, double w4) {
   constexpr double t13 = 13.0 / 12, eps = 1e-6, d0 = 1.0 / 16, d1 = 5.0 / 8, d2 = 5.0 / 16;
-  double v0 = 0.125 * (3 * v[0] - 10 * v[1] + 15 * v[2]);
-  double v1 = 0.125 * (-v[1] + 6 * v[2] + 3 * v[3]);
-  double v2 = 0.125 * (3 * v[2] + 6 * v[3] - v[4]);
-  double b0 = t13 * (v[0] + v[2] - 2 * v[1]) * (v[0] + v[2] - 2 * v[1]) +
-              0.25 * (v[0] + 3 * v[2] - 4 * v[1]) * (v[0] + 3 * v[2] - 4 * v[1]);
-  double b1 = t13 * (v[1] + v[3] - 2 * v[2]) * (v[1] + v[3] - 2 * v[2]) + 0.25 * (v[3] - v[1]) * (v[3] - v[1]);
-  double b2 = t13 * (v[2] + v[4] - 2 * v[3]) * (v[2] + v[4] - 2 * v[3]) +
-              0.25 * (3 * v[2] + v[4] - 4 * v[3]) * (3 * v[2] + v[4] - 4 * v[3]);
-  double tau = (b0 - b2) * (b0 - b2);
-  double a0 = d0 + d0 * tau / ((eps + b0) * (eps + b0));
-  double a1 = d1 + d1 * tau / ((eps + b1) * (eps + b1));
-  double a2 = d2 + d2 * tau / ((eps + b2) * (eps + b2));
-  vminus = (a0 * v0 + a1 * v1 + a2 * v2) / (a0 + a1 + a2);
-  v0 = v1;
-  v1 = v2;
-  v2 = 0.125 * (15 * v[3] - 10 * v[4] + 3 * v[5]);
-  b0 = t13 * (v[1] + v[3] - 2 * v[2]) * (v[1] + v[3] - 2 * v[2]) +
-       0.25 * (v[1] + 3 * v[3] - 4 * v[2]) * (v[1] + 3 * v[3] - 4 * v[2]);
-  b1 = t13 * (v[2] + v[4] - 2 * v[3]) * (v[2] + v[4] - 2 * v[3]) + 0.25 * (v[4] - v[2]) * (v[4] - v[2]);
-  b2 = t13 * (v[3] + v[5] - 2 * v[4]) * (v[3] + v[5] - 2 * v[4]) +
-       0.25 * (3 * v[3] + v[5] - 4 * v[4]) * (3 * v[3] + v[5] - 4 * v[4]);
-  tau = (b0 - b2) * (b0 - b2);
-  a0 = d2 + d2 * tau / ((eps + b0) * (eps + b0));
-  a1 = d1 + d1 * tau / ((eps + b1) * (eps + b1));
-  a2 = d0 + d0 * tau / ((eps + b2) * (eps + b2));
-  vplus = (a0 * v0 + a1 * v1 + a2 * v2) / (a0 + a1 + a2);
+  const double s0 = w0 + w2 - 2 * w1, s1 = w1 + w3 - 2 * w2, s2 = w2 + w4 - 2 * w3;
+  const double g0 = w0 + 3 * w2 - 4 * w1, g1 = w3 - w1, g2 = 3 * w2 + w4 - 4 * w3;
+  const double b0 = t13 * s0 * s0 + 0.25 * g0 * g0;
+  const double b1 = t13 * s1 * s1 + 0.25 * g1 * g1;
+  const double b2 = t13 * s2 * s2 + 0.25 * g2 * g2;
+  const double tau = (b0 - b2) * (b0 - b2);
+  const double e0 = (eps + b0) * (eps + b0), e1 = (eps + b1) * (eps + b1), e2 = (eps + b2) * (eps + b2);
+  const double a0 = d0 * (e0 + tau) * (e1 * e2), a1 = d1 * (e1 + tau) * (e0 * e2), a2 = d2 * (e2 + tau) * (e0 * e1);
+  const double v0 = 3 * w0 - 10 * w1 + 15 * w2, v1 = -w1 + 6 * w2 + 3 * w3, v2 = 3 * w2 + 6 * w3 - w4;
+  return 0.125 * (a0 * v0 + a1 * v1 + a2 * v2) / (a0 + a1 + a2);
+}
+__device__ __forceinline__ void weno5_pair(const double v[6], double &vminus, double &vplus) {
+  vminus = weno5(v[0], v[1], v[2], v[3], v[4]);
+  vplus = weno5(v[5], v[4], v[3], v[2], v[1]);
 }
 
 // NT = 2 (SST): k and omega are not part of the reference's AWENO (quirk A3:
@@ -534,23 +528,25 @@ __device__ __forceinline__ void inviscid_face_aweno(const DevZone &z, int g0, do
     for (int l = 0; l < 5; ++l) U[s][l] = cvl(z, g0 + (s - 2) * sd, l);
   const double pL = bvl(z, g0, 4), pR = bvl(z, g0 + sd, 4);
   const double *cl = U[2], *cr = U[3];
-  const double sl0 = sqrt(cl[0]), sr0 = sqrt(cr[0]);
-  const double rlc = sl0 / (sl0 + sr0), rrc = sr0 / (sl0 + sr0);
-  const double um = rlc * cl[1] / cl[0] + rrc * cr[1] / cr[0];
-  const double vm = rlc * cl[2] / cl[0] + rrc * cr[2] / cr[0];
-  const double wm = rlc * cl[3] / cl[0] + rrc * cr[3] / cr[0];
+  const double sl0 = sqrt(cl[0]), sr0 = sqrt(cr[0]), isum = 1.0 / (sl0 + sr0);
+  // Roe weights over the densities
+  const double wl = sl0 * isum / cl[0], wr = sr0 * isum / cr[0];
+  const double um = wl * cl[1] + wr * cr[1];
+  const double vm = wl * cl[2] + wr * cr[2];
+  const double wm = wl * cl[3] + wr * cr[3];
   const double ekm = 0.5 * (um * um + vm * vm + wm * wm);
-  const double hm = rlc * ((cl[4] + pL) / cl[0]) + rrc * ((cr[4] + pR) / cr[0]);
+  const double hm = wl * (cl[4] + pL) + wr * (cr[4] + pR);
   const double cm2 = gm1 * (hm - ekm);
   const double cm = sqrt(cm2);
+  const double ic2 = 1.0 / cm2, ic = cm * ic2, hc2 = 0.5 * ic2;
   const int g1 = g0 + sd;
   double kx = 0.5 * (met(z, g0, 3 * DIR) + met(z, g1, 3 * DIR));
   double ky = 0.5 * (met(z, g0, 3 * DIR + 1) + met(z, g1, 3 * DIR + 1));
   double kz = 0.5 * (met(z, g0, 3 * DIR + 2) + met(z, g1, 3 * DIR + 2));
-  const double gK = sqrt(kx * kx + ky * ky + kz * kz);
-  kx /= gK;
-  ky /= gK;
-  kz /= gK;
+  const double igK = 1.0 / sqrt(kx * kx + ky * ky + kz * kz);
+  kx *= igK;
+  ky *= igK;
+  kz *= igK;
   const double Uk = kx * um + ky * vm + kz * wm;
   const double alpha = gm1 * ekm;
   double ql[5] = {0, 0, 0, 0, 0}, qr[5] = {0, 0, 0, 0, 0};
@@ -560,39 +556,39 @@ __device__ __forceinline__ void inviscid_face_aweno(const DevZone &z, int g0, do
       double L[5];
       switch (r) {
         case 0:
-          L[0] = (alpha + Uk * cm) / cm2 * 0.5;
-          L[1] = -(gm1 * um + kx * cm) / cm2 * 0.5;
-          L[2] = -(gm1 * vm + ky * cm) / cm2 * 0.5;
-          L[3] = -(gm1 * wm + kz * cm) / cm2 * 0.5;
-          L[4] = gm1 / cm2 * 0.5;
+          L[0] = (alpha + Uk * cm) * hc2;
+          L[1] = -(gm1 * um + kx * cm) * hc2;
+          L[2] = -(gm1 * vm + ky * cm) * hc2;
+          L[3] = -(gm1 * wm + kz * cm) * hc2;
+          L[4] = gm1 * hc2;
           break;
         case 1:
-          L[0] = kx * (1 - alpha / cm2) - (kz * vm - ky * wm) / cm;
-          L[1] = kx * gm1 * um / cm2;
-          L[2] = (kx * gm1 * vm + kz * cm) / cm2;
-          L[3] = (kx * gm1 * wm - ky * cm) / cm2;
-          L[4] = -kx * gm1 / cm2;
+          L[0] = kx * (1 - alpha * ic2) - (kz * vm - ky * wm) * ic;
+          L[1] = kx * gm1 * um * ic2;
+          L[2] = (kx * gm1 * vm + kz * cm) * ic2;
+          L[3] = (kx * gm1 * wm - ky * cm) * ic2;
+          L[4] = -kx * gm1 * ic2;
           break;
         case 2:
-          L[0] = ky * (1 - alpha / cm2) - (kx * wm - kz * um) / cm;
-          L[1] = (ky * gm1 * um - kz * cm) / cm2;
-          L[2] = ky * gm1 * vm / cm2;
-          L[3] = (ky * gm1 * wm + kx * cm) / cm2;
-          L[4] = -ky * gm1 / cm2;
+          L[0] = ky * (1 - alpha * ic2) - (kx * wm - kz * um) * ic;
+          L[1] = (ky * gm1 * um - kz * cm) * ic2;
+          L[2] = ky * gm1 * vm * ic2;
+          L[3] = (ky * gm1 * wm + kx * cm) * ic2;
+          L[4] = -ky * gm1 * ic2;
           break;
         case 3:
-          L[0] = kz * (1 - alpha / cm2) - (ky * um - kx * vm) / cm;
-          L[1] = (kz * gm1 * um + ky * cm) / cm2;
-          L[2] = (kz * gm1 * vm - kx * cm) / cm2;
-          L[3] = kz * gm1 * wm / cm2;
-          L[4] = -kz * gm1 / cm2;
+          L[0] = kz * (1 - alpha * ic2) - (ky * um - kx * vm) * ic;
+          L[1] = (kz * gm1 * um + ky * cm) * ic2;
+          L[2] = (kz * gm1 * vm - kx * cm) * ic2;
+          L[3] = kz * gm1 * wm * ic2;
+          L[4] = -kz * gm1 * ic2;
           break;
         default:
-          L[0] = (alpha - Uk * cm) / cm2 * 0.5;
-          L[1] = -(gm1 * um - kx * cm) / cm2 * 0.5;
-          L[2] = -(gm1 * vm - ky * cm) / cm2 * 0.5;
-          L[3] = -(gm1 * wm - kz * cm) / cm2 * 0.5;
-          L[4] = gm1 / cm2 * 0.5;
+          L[0] = (alpha - Uk * cm) * hc2;
+          L[1] = -(gm1 * um - kx * cm) * hc2;
+          L[2] = -(gm1 * vm - ky * cm) * hc2;
+          L[3] = -(gm1 * wm - kz * cm) * hc2;
+          L[4] = gm1 * hc2;
       }
       double v[6];
 #pragma unroll
