@@ -720,25 +720,55 @@ void build_devparam(const ostc_param *p, DevParam &d) {
   }
 }
 
-// default tile shapes: enough CTAs for ~4 per SM, as few re-computed faces as possible
+// default tile shapes of a context's sweeps (before the autotuner or
+// ostc_set_tile choose). The build by what it is bound by, with flux times in us
+// of the x, y, z sweeps against the 255-register plane kernels that ran before:
+//  - staged where two CTAs fit an SM's shared memory, for mixtures (97 x 113 x 61,
+//    9 species: 253 / 313 / 315 against 549 / 760 / 737; 4 species 207 / 231 / 236
+//    against 231 / 310 / 306) and SST (9 blocks of air: 145 / 174 / 177 against
+//    264 / 375 / 400); one staged CTA per SM loses (12 species, y and z: 322 against
+//    267 for the 128-register plane kernel);
+//  - air: plane kernels of 80 registers (157 x 99 x 67: 114 / 131 / 143 against 165 /
+//    323 / 287, staged 139 / 147 / 148; Roe 147 / 173 / 182 against 220 / 444 / 393);
+//    a grid of one wave is latency-bound and takes 128 registers (41 x 33 x 10: 28
+//    against 32 for the three sweeps);
+//  - AWENO (no staged build, 240 registers wanted) and the rest: plane kernels of 128
+//    registers (128 x 96 x 80: 219 / 203 / 198 against 295 / 372 / 315).
+// Rows and chunks: a CTA takes about C + 0.15 chunk times (0.15: start-up and the
+// carried face), so the pair with the fewest waves times that wins.
 void default_tiles(ostc_ctx *c) {
-  const DevZone &z = c->dz[0];
-  int sms = 148;
-  int dev = 0;
+  int sms = 148, dev = 0;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long long target = 4ll * sms;
-  // x: rows 4, chunks so a segment spans the line, unless that leaves too few CTAs
-  {
-    int R = 4, C = (z.mx + 1 + 31) / 32;
-    while (C > 1 && (long long)((z.mx + 32 * C - 2) / (32 * C - 1)) * ((z.my + R - 1) / R) * z.mz < target) --C;
-    c->tile[0] = {R, std::max(C, 1), 1};
-  }
-  for (int d = 1; d < 3; ++d) {
-    const int n = d == 1 ? z.my : z.mz;
-    const int other = d == 1 ? z.mz : z.my;
-    int R = 8, C = (n + 1 + R - 1) / R;
-    while (C > 1 && (long long)((z.mx + 31) / 32) * other * ((n + R * C - 2) / (R * C - 1)) < target) --C;
-    c->tile[d] = {R, std::max(C, 1), 1};
+  const bool aweno = c->prm.inviscid_type == 1, roe = c->prm.inviscid_type == 2;
+  const bool viscous = c->prm.viscous_scheme != 0;
+  for (int d = 0; d < 3; ++d) {
+    auto tiles = [&](int R, int C) {
+      long long n = 0;
+      for (const DevZone &z : c->dz) {
+        const dim3 g = flux_grid(z.mx, z.my, z.mz, d, R, C);
+        n += (long long)g.x * g.y * g.z;
+      }
+      return n;
+    };
+    const size_t smem = stage_smem_bytes(c->ns, c->nt, d, viscous) + 64 * (5 + c->ns + c->nt) + 1024;
+    const bool staged = !aweno && ((c->ns > 0 && !roe) || c->nt > 0) && 2 * smem <= 228 * 1024;
+    const bool air80 = !aweno && c->ns == 0 && c->nt == 0 && tiles(8, 1) > 2 * sms;
+    TileShape best;
+    double cost = -1;
+    for (int R : {8, 4})
+      for (int C : {1, 2}) {
+        // staged CTAs have 8 rows, the 80-register plane CTAs 4; a 128-register CTA of one
+        // wave takes 8
+        if (R == 4 ? staged : air80) continue;
+        const long long slots = (long long)sms * (air80 ? 6 : (R == 8 ? 2 : 4));
+        const double w = (double)((tiles(R, C) + slots - 1) / slots) * (C + 0.15);
+        if (cost < 0 || w < cost) {
+          cost = w;
+          best = TileShape{R, C, air80 ? 3 : 2};
+          best.staged = staged;
+        }
+      }
+    c->tile[d] = best;
   }
 }
 
