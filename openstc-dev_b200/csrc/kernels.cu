@@ -1359,7 +1359,8 @@ cudaError_t launch_chem_surrogate(const mlp::Net &net, int n, const double *T, c
     chem_features_kernel<NS><<<cells_grid, 256, 0, s>>>(n, T, p, Y, dt, net.scale, net.checks, w.x, w.env);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     const int tiles = (n + tc::ROWS - 1) / tc::ROWS;
-    surrogate_chem_kernel<<<tiles < sms ? tiles : sms, tc::THREADS, tc::SM_BYTES, s>>>(net, w.x, w.y, n, w.err);
+    const int ctas = (tiles + tc::GROUPS - 1) / tc::GROUPS;
+    surrogate_chem_kernel<<<ctas < sms ? ctas : sms, tc::THREADS, tc::SM_BYTES, s>>>(net, w.x, w.y, n, w.err);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     chem_checks_kernel<NS><<<cells_grid, 256, 0, s>>>(n, T, Y, dt, w.y, w.env, net.scale, net.checks, dY, dT, w.list,
                                                       w.count);

@@ -287,17 +287,21 @@ unsigned blocks(long long n) { return (unsigned)((n + 255) / 256); }
 
 // the tensor-core forward on standardised rows (x [n][12] -> y [n][10])
 struct RawIo {
-  static constexpr bool kPacked = false;
   const float *x;
   float *y;
   int n;
-  __device__ void setup(unsigned char *) {}
-  __device__ bool load(int tile, int row, float *f) const {
-    const long long q = (long long)tile * tc::ROWS + row;
-    if (q >= n) return false;
+  __device__ void stage(int tile, unsigned char *x0, int t) const {
+    if (t >= tc::ROWS) return;
+    const long long q = (long long)tile * tc::ROWS + t;
+    float f[KIN] = {};
+    if (q < n)
 #pragma unroll
-    for (int i = 0; i < NIN; ++i) f[i] = x[q * NIN + i];
-    return true;
+      for (int i = 0; i < NIN; ++i) f[i] = x[q * NIN + i];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+      *(uint4 *)(x0 + tc::core_off(t, 8 * h, KIN)) =
+          make_uint4(tc::pack_bf16(f[8 * h], f[8 * h + 1]), tc::pack_bf16(f[8 * h + 2], f[8 * h + 3]),
+                     tc::pack_bf16(f[8 * h + 4], f[8 * h + 5]), tc::pack_bf16(f[8 * h + 6], f[8 * h + 7]));
   }
   __device__ void store(int tile, int row, const float *o) const {
     const long long q = (long long)tile * tc::ROWS + row;
@@ -656,7 +660,8 @@ ostc_status ostc_surrogate_forward_tc(ostc_surrogate *s, const float *xs, int n,
   SK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const int tiles = (n + tc::ROWS - 1) / tc::ROWS;
   SK(cudaMemsetAsync(s->err, 0, sizeof(int), st));
-  surrogate_raw_kernel<<<tiles < sms ? tiles : sms, tc::THREADS, tc::SM_BYTES, st>>>(s->net, xs, ys, n, s->err);
+  const int ctas = (tiles + tc::GROUPS - 1) / tc::GROUPS;
+  surrogate_raw_kernel<<<ctas < sms ? ctas : sms, tc::THREADS, tc::SM_BYTES, st>>>(s->net, xs, ys, n, s->err);
   SK(cudaGetLastError());
   int e = 0;
   SK(cudaMemcpyAsync(&e, s->err, sizeof(int), cudaMemcpyDeviceToHost, st));

@@ -81,11 +81,12 @@ __device__ __forceinline__ float energy_f(const ChemTables<NS> &tb, float t, con
   return e - (float)R_u * t * r;
 }
 
-// the scaling and acceptance tables of a CTA (thread 0 fills, the caller syncs)
+// the scaling and acceptance tables of a CTA (every thread fills its share, the
+// caller syncs; one thread alone took 9 us of each CTA)
 template <int NS>
 __device__ void fill_chem_tables(ChemTables<NS> *t, const double *scale, const mlp::Checks *ck) {
-  if (threadIdx.x != 0) return;
-  for (int i = 0; i < mlp::NIN; ++i) {
+  const int first = threadIdx.x, step = blockDim.x;
+  for (int i = first; i < mlp::NIN; i += step) {
     t->in_mean[i] = (float)scale[mlp::SC_IN_MEAN + i];
     t->in_istd[i] = (float)(1.0 / scale[mlp::SC_IN_STD + i]);
     // the envelope, widened by 1e-4 in log units so that the FP32 features
@@ -93,23 +94,24 @@ __device__ void fill_chem_tables(ChemTables<NS> *t, const double *scale, const m
     t->in_min[i] = __double2float_rd(scale[mlp::SC_IN_MIN + i] - 1e-4);
     t->in_max[i] = __double2float_ru(scale[mlp::SC_IN_MAX + i] + 1e-4);
   }
-  for (int l = 0; l < NS; ++l) {
-    for (int c = 0; c < 7; ++c) {
-      t->lo[l][c] = (float)c_p.lo[l][c];
-      t->hi[l][c] = (float)c_p.hi[l][c];
-    }
+  for (int e = first; e < NS * 7; e += step) {
+    const int l = e / 7, c = e % 7;
+    t->lo[l][c] = (float)c_p.lo[l][c];
+    t->hi[l][c] = (float)c_p.hi[l][c];
+  }
+  for (int l = first; l < NS; l += step) {
     t->t_low[l] = (float)c_p.t_low[l];
     t->t_mid[l] = (float)c_p.t_mid[l];
     t->Rmw[l] = (float)c_p.Rmw[l];
     t->imw[l] = (float)c_p.imw[l];
+    for (int e = 0; e < 4; ++e) t->a[e][l] = (float)ck->a[e][l];
   }
-  t->n_elem = ck->n_elem;
-  for (int e = 0; e < 4; ++e) {
-    t->m[e] = (float)ck->m[e];
-    for (int l = 0; l < NS; ++l) t->a[e][l] = (float)ck->a[e][l];
+  for (int e = first; e < 4; e += step) t->m[e] = (float)ck->m[e];
+  if (first == 0) {
+    t->n_elem = ck->n_elem;
+    t->tol_el = (float)ck->tol_el;
+    t->tol_T = (float)ck->tol_T;
   }
-  t->tol_el = (float)ck->tol_el;
-  t->tol_T = (float)ck->tol_T;
 }
 
 // stage 1 of the learned chemistry step, one thread per state: the FP32

@@ -1,22 +1,36 @@
 // tc_mlp.cuh — the surrogate network's forward pass on the 5th-generation
-// tensor cores (tcgen05): 128-row tiles, operands in shared memory in the
-// canonical no-swizzle K-major layout, FP32 accumulators in tensor memory.
+// tensor cores (tcgen05), transposed: the weights are the A operand and 64
+// states at a time the B operand, so that every weight stays on the SM.
 //
-// One CTA of 512 threads owns one SM (217 KB of shared memory) and walks
-// tiles of 128 rows. Per tile:
-//   features (FP64 -> standardised BF16, rows 0..127 by threads 0..127)
-//   L1  D[128x256]  = X0[128x16]  W1^T      1 MMA  (W1 resident)
-//   L2  D           = A1[128x256] W2^T     16 MMAs (W2 streamed from L2)
-//   L3  D           = A2          W3^T     16 MMAs (W3 streamed from L2)
-//   L4  D4[128x16]  = A3          W4^T     16 MMAs (W4 resident)
-// with the bias + SiLU + BF16 epilogues read from tensor memory by all 16
-// warps (warp w reads lanes 32 (w % 4).., columns 64 (w / 4)..). One
-// thread issues the MMAs and commits them to an mbarrier that every thread
-// waits on for at most WAIT_NS of the global timer. When a wait runs out
-// anywhere in the CTA, the whole CTA stops walking tiles: it sets the error
-// word, commits once more so that the barrier tracks every MMA it issued,
-// waits for that (bounded again) and for its own asynchronous copies, and
-// frees its tensor memory before it returns.
+// One CTA of 512 threads owns one SM: W2 (128 KB), W1 and W4 in shared memory,
+// W3 in half of tensor memory (an A operand may be read from there). Two groups
+// of 8 warps walk tiles of 64 states, each with its own activations (in place:
+// a layer's products are done before its epilogue writes) and its own 128
+// accumulator columns, so that the products of one group run under the
+// epilogue of the other. Per tile:
+//   L1  D[256x64]  = W1[256x16]  X0^T     2 MMAs (two halves of 128 features)
+//   L2  D          = W2[256x256] A1^T    32 MMAs (W2 from shared memory)
+//   L3  D          = W3[256x256] A2^T    32 MMAs (W3 from tensor memory)
+//   L4  D4[64x16]  = A3[64x256]  W4^T    16 MMAs (M = 128: the upper 64 rows read
+//                                        whatever follows the activations and
+//                                        are not used)
+// Epilogue: thread (warp, lane) holds one feature of all 64 states: bias, SiLU,
+// BF16 pairs of neighbouring features exchanged with the neighbouring lane, 4-byte
+// stores into the next layer's operand.
+//
+// Bound by the chain of a tile: three epilogues of 2400 cycles (the special-function
+// unit's share, 768 SiLUs a state at one exponential each and one reciprocal for two, is
+// 1536) and products of 2100 cycles a layer (66 cycles for each M = 128, N = 64, the rate of
+// N = 128), the two groups mostly in step. With 128-state tiles as the A operand, one in
+// flight per SM and W2 / W3 streamed from L2 for every tile, 1.5 million states took
+// 1718 us; now 1042.
+//
+// One thread of a group issues its MMAs and commits them to the group's mbarrier,
+// which the group waits on for at most WAIT_NS of the global timer. When a wait
+// runs out anywhere in a group, the group stops walking tiles: it sets the error
+// word, commits once more so that the barrier tracks every MMA it issued, waits
+// for that (bounded again) and for its own asynchronous copies; the CTA frees its
+// tensor memory when both groups are done.
 #pragma once
 #include <cuda_bf16.h>
 
@@ -29,21 +43,27 @@ using mlp::KIN;
 using mlp::NH;
 using mlp::NOUTP;
 
-constexpr int ROWS = 128;
-constexpr int THREADS = 512;
-// shared memory map (bytes)
-constexpr unsigned SM_ACT = 0;                       // 128 x 256 bf16
-constexpr unsigned SM_W = SM_ACT + ROWS * NH * 2;    // 256 x 256 bf16 (W2 or W3)
-constexpr unsigned SM_W1 = SM_W + NH * NH * 2;       // 256 x 16 bf16
-constexpr unsigned SM_W4 = SM_W1 + NH * KIN * 2;     // 16 x 256 bf16
-constexpr unsigned SM_X0 = SM_W4 + NOUTP * NH * 2;   // 128 x 16 bf16
-constexpr unsigned SM_BIAS = SM_X0 + ROWS * KIN * 2;  // b1, b2, b3 (FP32), b4 (16)
-constexpr unsigned SM_IO = SM_BIAS + (3 * NH + NOUTP) * 4;  // tables of the Io (IO_BYTES)
-constexpr unsigned IO_BYTES = 2048;
-constexpr unsigned SM_BAR = SM_IO + IO_BYTES;  // mbarrier (8 B)
-constexpr unsigned SM_TMEM = SM_BAR + 8;             // allocated tensor-memory base (4 B)
+constexpr int ROWS = 64;  // states per tile
+constexpr int THREADS = 512, GROUPS = 2, GTHREADS = THREADS / GROUPS;
+// activations of a tile as a K-major operand whose K-adjacent core matrices lie
+// 144 bytes apart: a warp's epilogue stores go to four of them at once, which at
+// the dense 128 bytes would share their banks
+constexpr unsigned ACT_LBO = 144, ACT_SBO = NH / 8 * ACT_LBO;
+constexpr unsigned ACT_BYTES = ROWS / 8 * ACT_SBO;
+// shared memory map (bytes); what follows the second activations is readable (layer 4)
+constexpr unsigned SM_ACT = 0;                                // 2 x 64 x 256 bf16
+constexpr unsigned SM_W2 = SM_ACT + GROUPS * ACT_BYTES;       // 256 x 256 bf16
+constexpr unsigned SM_W1 = SM_W2 + NH * NH * 2;               // 256 x 16 bf16
+constexpr unsigned SM_W4 = SM_W1 + NH * KIN * 2;              // 16 x 256 bf16
+constexpr unsigned SM_X0 = SM_W4 + NOUTP * NH * 2;            // 2 x 64 x 16 bf16
+constexpr unsigned SM_BAR = SM_X0 + GROUPS * ROWS * KIN * 2;  // one mbarrier (8 B) per group
+constexpr unsigned SM_TMEM = SM_BAR + 8 * GROUPS;             // allocated tensor-memory base (4 B)
 constexpr unsigned SM_BYTES = SM_TMEM + 8;
-constexpr unsigned TMEM_COLS = 512;
+static_assert(SM_BYTES <= 227 * 1024, "one CTA's shared memory");
+static_assert(SM_ACT + (GROUPS - 1) * ACT_BYTES + 128 / 8 * ACT_SBO <= SM_BYTES, "layer 4 reads 128 rows");
+// tensor memory: group g's accumulators in columns 128 g .. 128 g + 127 (64 per half
+// of the features), W3 in columns 256 .. 511 (128 per half)
+constexpr unsigned TMEM_COLS = 512, TM_W3 = 256;
 constexpr unsigned long long WAIT_NS = 1000000000ull;  // 1 s of the global timer per mbarrier wait
 
 // byte offset of element (r, k) of an R x K operand in the canonical K-major
@@ -90,19 +110,27 @@ __device__ __forceinline__ unsigned long long global_ns() {
   return t;
 }
 
-// bounded wait for the mbarrier phase `parity`; false when WAIT_NS ran out
+__device__ __forceinline__ bool bar_try(unsigned bar, unsigned parity) {
+  unsigned done;
+  asm volatile(
+      "{\n\t.reg .pred P;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
+      "selp.b32 %0, 1, 0, P;\n\t}\n"
+      : "=r"(done)
+      : "r"(bar), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+
+// bounded wait for the mbarrier phase `parity`; false when WAIT_NS ran out. The
+// timer is read only once a first round of tries has failed: the read is slow
+// against the products that most waits are for.
 __device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity) {
+  for (unsigned it = 0; it < 32; ++it)
+    if (bar_try(bar, parity)) return true;
   const unsigned long long t0 = global_ns();
   for (unsigned it = 0;; ++it) {
-    unsigned done;
-    asm volatile(
-        "{\n\t.reg .pred P;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 P, [%1], %2;\n\t"
-        "selp.b32 %0, 1, 0, P;\n\t}\n"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    if (done) return true;
+    if (bar_try(bar, parity)) return true;
     if ((it & 31) == 31 && global_ns() - t0 > WAIT_NS) return false;
   }
 }
@@ -173,163 +201,223 @@ __device__ __forceinline__ void load_weights(unsigned char *smem, unsigned off, 
   }
 }
 
-// The network core. `Io` supplies
-//   void setup(unsigned char *tables)          fills IO_BYTES of shared memory
-//                                              (all threads, once per CTA)
-// and, per tile, with Io::kPacked false
-//   bool load(int tile, int row, float *x12)   standardised features of a row
-//                                              (threads 0..127); false: no row
-// or with Io::kPacked true
-//   void stage(int tile, unsigned char *x0)    all threads: the tile's rows,
-//                                              already standardised BF16, into
-//                                              the operand layout (cp.async)
-// and
+// one MMA with the A operand in tensor memory
+__device__ __forceinline__ void mma_issue_ta(unsigned tmem_d, unsigned tmem_a, unsigned long long b, unsigned idesc,
+                                             unsigned accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}\n" ::"r"(tmem_d),
+      "r"(tmem_a), "l"(b), "r"(idesc), "r"(accumulate));
+}
+
+// 32 consecutive columns of this thread's lane, written (no wait: tmem_wait_st)
+__device__ __forceinline__ void tmem_st32(unsigned taddr, const unsigned *r) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
+      "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};\n" ::"r"(taddr),
+      "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+      "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]), "r"(r[16]), "r"(r[17]), "r"(r[18]),
+      "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]), "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]),
+      "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
+// the barrier of one group's threads, and the same with an OR over them
+__device__ __forceinline__ void group_sync(int g) {
+  asm volatile("barrier.cta.sync %0, %1;" ::"r"(1 + g), "r"(GTHREADS) : "memory");
+}
+__device__ __forceinline__ bool group_or(int g, bool v) {
+  unsigned r;
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.u32 p, %1, 0;\n\t"
+      "barrier.cta.red.or.pred q, %2, %3, p;\n\t"
+      "selp.u32 %0, 1, 0, q;\n\t}\n"
+      : "=r"(r)
+      : "r"((unsigned)v), "r"(1 + g), "r"(GTHREADS)
+      : "memory");
+  return r != 0;
+}
+
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+// z / (1 + exp(-z)) of two values with one reciprocal; the exponentials are held
+// below 2^62, so that the product of the denominators stays finite (SiLU is below
+// 1e-16 there)
+__device__ __forceinline__ void silu2(float &a, float &b) {
+  constexpr float log2e = 1.4426950408889634f;
+  const float da = 1.f + ex2(fminf(-log2e * a, 62.f)), db = 1.f + ex2(fminf(-log2e * b, 62.f));
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(da * db));
+  a *= r * db;
+  b *= r * da;
+}
+
+// The network core. `Io` supplies, per tile of 64 rows and for the group's threads
+// (t = 0 .. 255),
+//   void stage(int tile, unsigned char *x0, int t)    the tile's rows as standardised
+//                                              BF16 in the operand layout, by plain
+//                                              stores or cp.async
 //   void store(int tile, int row, const float *y10)   standardised outputs
 // Returns nothing; errors go to *err (1 = a wait ran out).
 template <typename Io>
 __device__ void mlp_tiles(const mlp::Net &net, int n_tiles, Io &io, int *err) {
   extern __shared__ __align__(1024) unsigned char smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const unsigned bar = smem_u32(smem + SM_BAR);
+  const int g = tid / GTHREADS, t = tid % GTHREADS;  // group, thread of the group
+  const int half = (warp >> 2) & 1;                  // features 128 half .. 128 half + 127
+  const int f = half * 128 + (warp & 3) * 32 + lane;  // this thread's feature
+  const unsigned bar = smem_u32(smem + SM_BAR + 8 * g);
   unsigned *tmem_slot = (unsigned *)(smem + SM_TMEM);
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                  "r"(TMEM_COLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
   }
-  if (tid == 0) {
+  if (t == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  // resident weights and biases
+  // resident weights; each thread keeps its feature's biases
   load_weights(smem, SM_W1, net.w1(), NH, KIN);
+  load_weights(smem, SM_W2, net.w2(), NH, NH);
   load_weights(smem, SM_W4, net.w4(), NOUTP, NH);
-  float *sbias = (float *)(smem + SM_BIAS);
-  for (int c = tid; c < NH; c += THREADS) {
-    sbias[c] = net.b1()[c];
-    sbias[NH + c] = net.b2()[c];
-    sbias[2 * NH + c] = net.b3()[c];
+  const float bias1 = net.b1()[f], bias2 = net.b2()[f], bias3 = net.b3()[f];
+  fence_before();
+  __syncthreads();
+  fence_after();
+  const unsigned tmem = *tmem_slot;
+  const unsigned lane_addr = (unsigned)((warp & 3) * 32) << 16;
+  if (g == 0) {  // W3: row f into lane f % 128, two values of K per column
+    const uint4 *w = (const uint4 *)(net.w3() + (long long)f * NH);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      unsigned r[32];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const uint4 v = __ldg(w + c * 8 + e);
+        r[4 * e] = v.x, r[4 * e + 1] = v.y, r[4 * e + 2] = v.z, r[4 * e + 3] = v.w;
+      }
+      tmem_st32(tmem + lane_addr + TM_W3 + half * 128 + c * 32, r);
+    }
+    tmem_wait_st();
   }
-  if (tid < NOUTP) sbias[3 * NH + tid] = net.b4()[tid];
-  io.setup(smem + SM_IO);
   cp_async_wait_all();
   fence_async_smem();
   fence_before();
   __syncthreads();
   fence_after();
-  const unsigned tmem = *tmem_slot;
-  const unsigned tmem_d4 = tmem + NH;  // columns 256..271
-  unsigned parity = 0;
-  bool timed_out = false;  // CTA-uniform: a bounded wait ran out somewhere in the CTA
-  const int row = (warp & 3) * 32 + lane;   // the TMEM lane this thread reads
-  const int col0 = (warp >> 2) * (NH / 4);  // first of its 64 columns
-  const unsigned lane_addr = (unsigned)((warp & 3) * 32) << 16;
 
-  for (int tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-    if constexpr (Io::kPacked) {
-      // the tile's feature rows first, then W2, which streams during layer 1
-      io.stage(tile, smem + SM_X0);
-      cp_async_commit();
-      load_weights(smem, SM_W, net.w2(), NH, NH);
-      cp_async_commit();
-      cp_async_wait_prior1();
-    } else {
-    // stream W2 while the features and layer 1 run
-    load_weights(smem, SM_W, net.w2(), NH, NH);
-    if (tid < ROWS) {
-      float x[12];
-      const bool has = io.load(tile, tid, x);
-      float xs[16];
-#pragma unroll
-      for (int i = 0; i < 12; ++i) xs[i] = has ? x[i] : 0.f;
-#pragma unroll
-      for (int i = 12; i < 16; ++i) xs[i] = 0.f;
-      *(uint4 *)(smem + SM_X0 + core_off(tid, 0, KIN)) = make_uint4(
-          pack_bf16(xs[0], xs[1]), pack_bf16(xs[2], xs[3]), pack_bf16(xs[4], xs[5]), pack_bf16(xs[6], xs[7]));
-      *(uint4 *)(smem + SM_X0 + core_off(tid, 8, KIN)) = make_uint4(
-          pack_bf16(xs[8], xs[9]), pack_bf16(xs[10], xs[11]), pack_bf16(xs[12], xs[13]), pack_bf16(xs[14], xs[15]));
-    }
-    }
+  unsigned char *act = smem + SM_ACT + g * ACT_BYTES, *x0 = smem + SM_X0 + g * ROWS * KIN * 2;
+  const unsigned act0 = smem_u32(act), d0 = tmem + 128 * g;
+  // where this thread's stores go: even lanes hold the even states of a pair of
+  // features, odd lanes the odd ones
+  unsigned char *out = act + (f >> 3) * ACT_LBO + (f & 6) * 2 + (lane & 1) * 16;
+  unsigned parity = 0;
+  bool timed_out = false;  // group-uniform: a bounded wait ran out somewhere in the group
+  const int stride = GROUPS * gridDim.x;
+  int tile = blockIdx.x * GROUPS + g;
+  if (tile < n_tiles) io.stage(tile, x0, t);
+  for (; tile < n_tiles; tile += stride) {
+    cp_async_wait_all();
     fence_async_smem();
     fence_before();
-    __syncthreads();
+    group_sync(g);
     fence_after();
-    if (tid == 0) {
-      mma_issue(tmem, smem_desc(smem_u32(smem + SM_X0), 128, 2 * 128), smem_desc(smem_u32(smem + SM_W1), 128, 2 * 128),
-                idesc_bf16(NH), 0);
+    if (t == 0) {
+      const unsigned long long b = smem_desc(smem_u32(x0), 128, 2 * 128);
+      for (int h = 0; h < 2; ++h)
+        mma_issue(d0 + 64 * h, smem_desc(smem_u32(smem + SM_W1) + h * 128 * KIN * 2, 128, 2 * 128), b, idesc_bf16(ROWS),
+                  0);
       // net.withhold_commit (a diagnostic of the timeout path): no completion
       // signal for this product, so the wait below runs out
       if (!net.withhold_commit) mma_commit(bar);
     }
     for (int layer = 0; layer < 3; ++layer) {
-      if (__syncthreads_or(!bar_wait(bar, parity))) {
+      if (group_or(g, !bar_wait(bar, parity))) {
         timed_out = true;
         break;
       }
       parity ^= 1;
       fence_after();
-      if (layer == 1) load_weights(smem, SM_W, net.w3(), NH, NH);  // W2 is no longer read
-      // epilogue: bias + SiLU -> BF16 activations (the next layer's A operand)
-      const float *b = sbias + layer * NH;
-      // both 32-column loads in flight before the one wait
-      unsigned acc[NH / 4];
-      tmem_ld32_async(tmem + lane_addr + col0, acc);
-      tmem_ld32_async(tmem + lane_addr + col0 + 32, acc + 32);
+      // the next tile's rows load under this tile's layers (layer 1 has read its own)
+      if (layer == 0 && tile + stride < n_tiles) io.stage(tile + stride, x0, t);
+      // epilogue: bias + SiLU -> BF16 activations (the next layer's operand)
+      const float b = layer == 0 ? bias1 : (layer == 1 ? bias2 : bias3);
+      unsigned acc[ROWS];
+      tmem_ld32_async(d0 + lane_addr + 64 * half, acc);
+      tmem_ld32_async(d0 + lane_addr + 64 * half + 32, acc + 32);
       tmem_wait_ld();
 #pragma unroll
-      for (int q = 0; q < NH / 4; q += 8) {
-        const float4 b0 = *(const float4 *)(b + col0 + q), b1 = *(const float4 *)(b + col0 + q + 4);
-        const float bb[8] = {b0.x, b0.y, b0.z, b0.w, b1.x, b1.y, b1.z, b1.w};
-        unsigned w4[4];
-#pragma unroll
-        for (int e = 0; e < 8; e += 2) {
-          const float z0 = __uint_as_float(acc[q + e]) + bb[e], z1 = __uint_as_float(acc[q + e + 1]) + bb[e + 1];
-          w4[e / 2] = pack_bf16(__fdividef(z0, 1.0f + __expf(-z0)), __fdividef(z1, 1.0f + __expf(-z1)));
-        }
-        *(uint4 *)(smem + SM_ACT + core_off(row, col0 + q, NH)) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
+      for (int n = 0; n < ROWS; n += 2) {
+        float a0 = __uint_as_float(acc[n]) + b, a1 = __uint_as_float(acc[n + 1]) + b;
+        silu2(a0, a1);
+        const unsigned own = pack_bf16(a0, a1);  // states n, n + 1 of this feature
+        const unsigned oth = __shfl_xor_sync(0xffffffffu, own, 1);
+        // even lane: state n of features f, f + 1; odd lane: state n + 1 of f - 1, f
+        const unsigned w = lane & 1 ? __byte_perm(oth, own, 0x7632) : __byte_perm(own, oth, 0x5410);
+        *(unsigned *)(out + (n >> 3) * ACT_SBO + (n & 7) * 16) = w;
       }
-      cp_async_wait_all();
       fence_async_smem();
       fence_before();
-      __syncthreads();
+      group_sync(g);
       fence_after();
-      if (tid == 0) {
-        const unsigned a0 = smem_u32(smem + SM_ACT);
-        const unsigned w0 = smem_u32(smem + (layer < 2 ? SM_W : SM_W4));
-        const unsigned d = layer < 2 ? tmem : tmem_d4;
-        const unsigned id = idesc_bf16(layer < 2 ? NH : NOUTP);
-        for (int s = 0; s < NH / 16; ++s)
-          mma_issue(d, smem_desc(a0 + s * 256, 128, NH * 16), smem_desc(w0 + s * 256, 128, NH * 16), id, s > 0);
+      if (t == 0) {
+        // unrolled, so that each product costs its one thread an addition per descriptor
+        const unsigned long long ad = smem_desc(act0, ACT_LBO, ACT_SBO);
+        constexpr unsigned id = idesc_bf16(ROWS);
+        if (layer == 0) {
+          const unsigned long long wd = smem_desc(smem_u32(smem + SM_W2), 128, NH * 16);
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int s = 0; s < NH / 16; ++s)
+              mma_issue(d0 + 64 * h, wd + (h * 128 * NH * 2 + s * 256) / 16, ad + s * 2 * ACT_LBO / 16, id, s > 0);
+        } else if (layer == 1) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int s = 0; s < NH / 16; ++s)
+              mma_issue_ta(d0 + 64 * h, tmem + TM_W3 + h * 128 + s * 8, ad + s * 2 * ACT_LBO / 16, id, s > 0);
+        } else {
+          const unsigned long long wd = smem_desc(smem_u32(smem + SM_W4), 128, NH * 16);
+#pragma unroll
+          for (int s = 0; s < NH / 16; ++s)
+            mma_issue(d0, ad + s * 2 * ACT_LBO / 16, wd + s * 256 / 16, idesc_bf16(NOUTP), s > 0);
+        }
         mma_commit(bar);
       }
     }
-    if (timed_out || __syncthreads_or(!bar_wait(bar, parity))) {
+    if (timed_out || group_or(g, !bar_wait(bar, parity))) {
       timed_out = true;
       break;
     }
     parity ^= 1;
     fence_after();
-    if (warp < 4) {
+    if (t < ROWS) {
       float v[16], y[10];
-      tmem_ld16(tmem_d4 + lane_addr, v);
+      tmem_ld16(d0 + lane_addr, v);
 #pragma unroll
-      for (int i = 0; i < 10; ++i) y[i] = v[i] + sbias[3 * NH + i];
-      io.store(tile, row, y);
+      for (int i = 0; i < 10; ++i) y[i] = v[i] + net.b4()[i];
+      io.store(tile, t, y);
     }
-    fence_before();
-    __syncthreads();
-    fence_after();
   }
   if (timed_out) {
-    // drain: one more commit tracks every MMA this CTA issued; wait for it
-    // (bounded) and for the CTA's own weight copies before the memory goes
-    if (tid == 0) {
+    // drain: one more commit tracks every MMA this group issued; wait for it
+    // (bounded) before the memory goes
+    if (t == 0) {
       mma_commit(bar);
       if (err) atomicExch(err, 1);
     }
     bar_wait(bar, parity);
-    cp_async_wait_all();
   }
+  cp_async_wait_all();
   fence_before();
   __syncthreads();
   fence_after();
@@ -339,21 +427,18 @@ __device__ void mlp_tiles(const mlp::Net &net, int n_tiles, Io &io, int *err) {
 // rows of 16 standardised BF16 features (12 and 4 zeros, 32 bytes, the
 // operand's K) in; rows of 10 FP32 outputs out
 struct PackedIo {
-  static constexpr bool kPacked = true;
   const __nv_bfloat16 *x;
   float *y;
   int n;
-  __device__ void setup(unsigned char *) {}
-  __device__ void stage(int tile, unsigned char *x0) const {
-    for (int c = threadIdx.x; c < 2 * ROWS; c += THREADS) {
-      const int row = c >> 1, half = c & 1;
-      const long long q = (long long)tile * ROWS + row;
-      unsigned char *dst = x0 + core_off(row, half * 8, KIN);
-      if (q < n)
-        cp_async16(smem_u32(dst), x + q * KIN + half * 8);
-      else
-        *(uint4 *)dst = make_uint4(0, 0, 0, 0);
-    }
+  __device__ void stage(int tile, unsigned char *x0, int t) const {
+    if (t >= 2 * ROWS) return;
+    const int row = t >> 1, half = t & 1;
+    const long long q = (long long)tile * ROWS + row;
+    unsigned char *dst = x0 + core_off(row, half * 8, KIN);
+    if (q < n)
+      cp_async16(smem_u32(dst), x + q * KIN + half * 8);
+    else
+      *(uint4 *)dst = make_uint4(0, 0, 0, 0);
   }
   __device__ void store(int tile, int row, const float *o) const {
     const long long q = (long long)tile * ROWS + row;
