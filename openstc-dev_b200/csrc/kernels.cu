@@ -432,93 +432,162 @@ static __global__ void dt_reset_kernel(unsigned long long *dt_bits) {
 
 // ---------------------------------------------------------------------------
 // boundary conditions. One thread per boundary point of the face range.
+//
+// A point's primitive state and scalars are read into registers first and
+// written from there, the conservative values computed from the registers
+// too: a load that follows a store to memory which may be its own waits for
+// it, so that copying plane by plane was a chain of 15 to 50 round trips per
+// point (a wave of small faces took 15 us).
 // ---------------------------------------------------------------------------
+template <int NS>
+struct PointState {
+  double b[6], y[NS + 2], mut;  // rho, u, v, w, p, T; species and (SST) k, omega; mut
+};
+
+template <int NS>
+__device__ __forceinline__ void load_point(const DevZone &z, int g, PointState<NS> &s) {
+#pragma unroll
+  for (int l = 0; l < 6; ++l) s.b[l] = z.bv[l * z.sz + g];
+#pragma unroll
+  for (int l = 0; l < NS + 2; ++l) s.y[l] = l < c_p.n_scalar ? z.sv[l * z.sz + g] : 0.0;
+  s.mut = c_p.sst ? z.mut[g] : 0.0;
+}
+
+template <int NS>
+__device__ __forceinline__ void store_point(const DevZone &z, int g, const PointState<NS> &s, bool mut = true) {
+#pragma unroll
+  for (int l = 0; l < 6; ++l) z.bv[l * z.sz + g] = s.b[l];
+#pragma unroll
+  for (int l = 0; l < NS + 2; ++l)
+    if (l < c_p.n_scalar) z.sv[l * z.sz + g] = s.y[l];
+  if (mut && c_p.sst) z.mut[g] = s.mut;
+}
+
+// the total energy of a state, as cv_from_bv_point forms it
+template <int NS>
+__device__ __forceinline__ double point_energy(const PointState<NS> &s, double V2) {
+  double E = 0.5 * V2;
+  if constexpr (NS == 0) {
+    E *= s.b[0];
+    E += s.b[4] / (gamma_air - 1);
+  } else {
+    double h[NS];
+    enthalpy<NS>(s.b[5], h);
+#pragma unroll
+    for (int l = 0; l < NS; ++l) E += h[l] * s.y[l];
+    E *= s.b[0];
+    E -= s.b[4];
+  }
+  return E;
+}
+
+// conservative values and velocity of a state with energy E (cv_from_bv_point)
+template <int NS>
+__device__ __forceinline__ void store_cv(const DevZone &z, int g, const PointState<NS> &s, double V2, double E) {
+  z.cv[g] = s.b[0];
+#pragma unroll
+  for (int d = 1; d < 4; ++d) z.cv[d * z.sz + g] = s.b[0] * s.b[d];
+  z.cv[4 * z.sz + g] = E;
+#pragma unroll
+  for (int l = 0; l < NS + 2; ++l)
+    if (l < c_p.n_scalar) z.cv[(5 + l) * z.sz + g] = s.b[0] * s.y[l];
+  z.vel[g] = sqrt(V2);
+}
+template <int NS>
+__device__ __forceinline__ void store_cv(const DevZone &z, int g, const PointState<NS> &s) {
+  const double V2 = s.b[1] * s.b[1] + s.b[2] * s.b[2] + s.b[3] * s.b[3];
+  store_cv<NS>(z, g, s, V2, point_energy<NS>(s, V2));
+}
+
+// the same state into the ngg layers outward of g
+template <int NS>
+__device__ __forceinline__ void extrapolate_point(const DevZone &z, int g, int step, int first, const PointState<NS> &s,
+                                                  int with_cv) {
+  const double V2 = s.b[1] * s.b[1] + s.b[2] * s.b[2] + s.b[3] * s.b[3];
+  const double E = with_cv ? point_energy<NS>(s, V2) : 0.0;
+  for (int gg = first; gg <= z.ngg; ++gg) {
+    store_point<NS>(z, g + gg * step, s);
+    if (with_cv) store_cv<NS>(z, g + gg * step, s, V2, E);
+  }
+}
+
 template <int NS>
 __device__ __forceinline__ void bc_outflow_point(const DevZone &z, const BcFace &b, int with_cv, int i, int j, int k) {  // BoundCond.cuh:120-150
   const int g = gidx(z, i, j, k);
-  const int step = b.dir_stride;
-  for (int gg = 1; gg <= z.ngg; ++gg) {
-    const int gi = g + gg * step;
-    for (int l = 0; l < 6; ++l) z.bv[l * z.sz + gi] = z.bv[l * z.sz + g];
-    for (int l = 0; l < c_p.n_scalar; ++l) z.sv[l * z.sz + gi] = z.sv[l * z.sz + g];
-    if (c_p.sst) z.mut[gi] = z.mut[g];
-    if (with_cv) cv_from_bv_point<NS>(z, gi);
-  }
+  PointState<NS> s;
+  load_point<NS>(z, g, s);
+  extrapolate_point<NS>(z, g, b.dir_stride, 1, s, with_cv);
 }
 
 template <int NS>
 __device__ __forceinline__ void bc_inflow_point(const DevZone &z, const BcFace &b, int with_cv, int i, int j, int k) {  // BoundCond.cuh:152-210
   const int g = gidx(z, i, j, k);
-  const int step = b.dir_stride;
-  for (int gg = 0; gg <= z.ngg; ++gg) {
-    const int gi = g + gg * step;
-    z.bv[gi] = b.density;
-    z.bv[z.sz + gi] = b.u;
-    z.bv[2 * z.sz + gi] = b.v;
-    z.bv[3 * z.sz + gi] = b.w;
-    z.bv[4 * z.sz + gi] = b.pressure;
-    z.bv[5 * z.sz + gi] = b.temperature;
-    for (int l = 0; l < c_p.n_scalar; ++l) z.sv[l * z.sz + gi] = b.sv[l];
-    if (c_p.sst) z.mut[gi] = b.mut;
-    if (gg == 0) z.vel[gi] = b.velocity;
-    if (with_cv) {
-      // compute_cv_from_bv_1_point also rewrites vel from bv (FieldOperation.cuh:40)
-      cv_from_bv_point<NS>(z, gi);
-    }
-  }
+  PointState<NS> s;
+  s.b[0] = b.density;
+  s.b[1] = b.u;
+  s.b[2] = b.v;
+  s.b[3] = b.w;
+  s.b[4] = b.pressure;
+  s.b[5] = b.temperature;
+#pragma unroll
+  for (int l = 0; l < NS + 2; ++l) s.y[l] = l < c_p.n_scalar ? b.sv[l] : 0.0;
+  s.mut = b.mut;
+  // compute_cv_from_bv_1_point also rewrites vel from bv (FieldOperation.cuh:40)
+  if (!with_cv) z.vel[g] = b.velocity;
+  extrapolate_point<NS>(z, g, b.dir_stride, 0, s, with_cv);
 }
 
-static __device__ __forceinline__ void bc_symmetry_point(const DevZone &z, const BcFace &b, int, int i, int j, int k) {  // BoundCond.cuh:52-118
+template <int NS>
+__device__ __forceinline__ void bc_symmetry_point(const DevZone &z, const BcFace &b, int, int i, int j, int k) {  // BoundCond.cuh:52-118
   const int g = gidx(z, i, j, k);
   const int step = b.dir_stride;
-  const int gin = g - step;
   double kx = z.met[(3 * b.face) * z.sz + g], ky = z.met[(3 * b.face + 1) * z.sz + g];
   double kz = z.met[(3 * b.face + 2) * z.sz + g];
+  PointState<NS> s;
+  load_point<NS>(z, g - step, s);
   const double km = sqrt(kx * kx + ky * ky + kz * kz);
   kx /= km;
   ky /= km;
   kz /= km;
-  const double u1 = z.bv[z.sz + gin], v1 = z.bv[2 * z.sz + gin], w1 = z.bv[3 * z.sz + gin];
-  double uk = kx * u1 + ky * v1 + kz * w1;
-  const double ut = u1 - kx * uk, vt = v1 - ky * uk, wt = w1 - kz * uk;
-  z.bv[z.sz + g] = ut;
-  z.bv[2 * z.sz + g] = vt;
-  z.bv[3 * z.sz + g] = wt;
-  z.vel[g] = sqrt(ut * ut + vt * vt + wt * wt);
-  z.bv[g] = z.bv[gin];
-  z.bv[4 * z.sz + g] = z.bv[4 * z.sz + gin];
-  z.bv[5 * z.sz + g] = z.bv[5 * z.sz + gin];
-  for (int l = 0; l < c_p.n_scalar; ++l) z.sv[l * z.sz + g] = z.sv[l * z.sz + gin];
-  for (int gg = 1; gg <= z.ngg; ++gg) {
-    const int go = g + gg * step, gi = g - gg * step;
-    z.bv[go] = z.bv[gi];
-    const double u = z.bv[z.sz + gi], v = z.bv[2 * z.sz + gi], w = z.bv[3 * z.sz + gi];
-    uk = kx * u + ky * v + kz * w;
-    const double uo = u - 2 * uk * kx, vo = v - 2 * uk * ky, wo = w - 2 * uk * kz;
-    z.bv[z.sz + go] = uo;
-    z.bv[2 * z.sz + go] = vo;
-    z.bv[3 * z.sz + go] = wo;
-    z.vel[go] = sqrt(uo * uo + vo * vo + wo * wo);
-    z.bv[4 * z.sz + go] = z.bv[4 * z.sz + gi];
-    z.bv[5 * z.sz + go] = z.bv[5 * z.sz + gi];
-    for (int l = 0; l < c_p.n_scalar; ++l) z.sv[l * z.sz + go] = z.sv[l * z.sz + gi];
-    if (c_p.sst) z.mut[go] = z.mut[gi];
+  // the boundary point takes the first inner point's state without its normal
+  // velocity, ghost layer gg the mirror image of the gg-th inner point
+  for (int gg = 0; gg <= z.ngg; ++gg) {
+    PointState<NS> nx;  // the next layer's source, read before this layer is written
+    if (gg >= 1 && gg < z.ngg) load_point<NS>(z, g - (gg + 1) * step, nx);
+    PointState<NS> o = s;
+    const double u = s.b[1], v = s.b[2], w = s.b[3];
+    const double uk = kx * u + ky * v + kz * w;
+    if (gg == 0) {
+      o.b[1] = u - kx * uk, o.b[2] = v - ky * uk, o.b[3] = w - kz * uk;
+    } else {
+      o.b[1] = u - 2 * uk * kx, o.b[2] = v - 2 * uk * ky, o.b[3] = w - 2 * uk * kz;
+    }
+    const int go = g + gg * step;
+    store_point<NS>(z, go, o, gg > 0);  // mut in the ghosts only
+    z.vel[go] = sqrt(o.b[1] * o.b[1] + o.b[2] * o.b[2] + o.b[3] * o.b[3]);
+    if (gg >= 1) s = nx;
   }
 }
 
 // periodic wrap (no reference counterpart): ghost layer gg of this face takes
 // the point n cells back along the face normal
-static __device__ __forceinline__ void bc_periodic_point(const DevZone &z, const BcFace &b, int with_cv, int i, int j, int k) {
+template <int NS>
+__device__ __forceinline__ void bc_periodic_point(const DevZone &z, const BcFace &b, int with_cv, int i, int j, int k) {
   const int g = gidx(z, i, j, k);
   for (int gg = 1; gg <= z.ngg; ++gg) {
     const int go = g + gg * b.dir_stride;
     const int gs = go - b.period_stride;
-    for (int l = 0; l < 6; ++l) z.bv[l * z.sz + go] = z.bv[l * z.sz + gs];
-    for (int l = 0; l < c_p.n_scalar; ++l) z.sv[l * z.sz + go] = z.sv[l * z.sz + gs];
-    if (c_p.sst) z.mut[go] = z.mut[gs];
-    z.vel[go] = z.vel[gs];
-    if (with_cv)
-      for (int l = 0; l < c_p.n_var; ++l) z.cv[l * z.sz + go] = z.cv[l * z.sz + gs];
+    PointState<NS> s;
+    double c[NS + 7];
+    load_point<NS>(z, gs, s);
+    const double vel = z.vel[gs];
+#pragma unroll
+    for (int l = 0; l < NS + 7; ++l) c[l] = with_cv && l < c_p.n_var ? z.cv[l * z.sz + gs] : 0.0;
+    store_point<NS>(z, go, s);
+    z.vel[go] = vel;
+#pragma unroll
+    for (int l = 0; l < NS + 7; ++l)
+      if (with_cv && l < c_p.n_var) z.cv[l * z.sz + go] = c[l];
   }
 }
 
@@ -567,36 +636,33 @@ __device__ __forceinline__ void bc_wall_point(const DevZone &z, const BcFace &b,
         dy > 1e-25 ? 60 * mu_wall / (rho_wall * sst::beta_1 * dy * dy) : z.sv[(NS + 1) * z.sz + gin];
   }
   if (with_cv) cv_from_bv_point<NS>(z, g);
+  const double om_w = c_p.sst ? z.sv[(NS + 1) * z.sz + g] : 0.0;
   for (int gg = 1; gg <= z.ngg; ++gg) {
     const int gi = g - gg * step, go = g + gg * step;
-    const double u_i = z.bv[z.sz + gi], v_i = z.bv[2 * z.sz + gi], w_i = z.bv[3 * z.sz + gi];
-    const double p_i = z.bv[4 * z.sz + gi], t_i = z.bv[5 * z.sz + gi];
-    double t_g = t_i;
+    PointState<NS> s;
+    load_point<NS>(z, gi, s);
+    double t_g = s.b[5];
     if (b.wall_isothermal) {
-      t_g = 2 * t_wall - t_i;
+      t_g = 2 * t_wall - t_g;
       if (t_g <= 0.1 * t_wall) t_g = t_wall;
     }
     if constexpr (NS > 0) {
       mw = 0;
 #pragma unroll
-      for (int l = 0; l < NS; ++l) {
-        z.sv[l * z.sz + go] = z.sv[l * z.sz + gi];
-        mw += z.sv[l * z.sz + go] * c_p.imw[l];
-      }
+      for (int l = 0; l < NS; ++l) mw += s.y[l] * c_p.imw[l];
       mw = 1 / mw;
     }
-    z.bv[go] = p_i * mw / (t_g * R_u);
-    z.bv[z.sz + go] = -u_i;
-    z.bv[2 * z.sz + go] = -v_i;
-    z.bv[3 * z.sz + go] = -w_i;
-    z.bv[4 * z.sz + go] = p_i;
-    z.bv[5 * z.sz + go] = t_g;
+    s.b[0] = s.b[4] * mw / (t_g * R_u);
+#pragma unroll
+    for (int d = 1; d < 4; ++d) s.b[d] = -s.b[d];
+    s.b[5] = t_g;
     if (c_p.sst) {
-      z.sv[NS * z.sz + go] = 0;
-      z.sv[(NS + 1) * z.sz + go] = z.sv[(NS + 1) * z.sz + g];
-      z.mut[go] = 0;
+      s.y[NS] = 0;
+      s.y[NS + 1] = om_w;
+      s.mut = 0;
     }
-    if (with_cv) cv_from_bv_point<NS>(z, go);
+    store_point<NS>(z, go, s);
+    if (with_cv) store_cv<NS>(z, go, s);
   }
 }
 
@@ -649,12 +715,9 @@ __device__ __forceinline__ void bc_farfield_point(const DevZone &z, const BcFace
   if (mach_b <= -1) {
     fill(b.density, b.u, b.v, b.w, b.pressure, b.temperature, b.sv, b.mut, true);
   } else if (mach_b >= 1) {
-    for (int gg = 1; gg <= z.ngg; ++gg) {
-      const int go = g + gg * step;
-      for (int l = 0; l < 6; ++l) z.bv[l * z.sz + go] = z.bv[l * z.sz + g];
-      for (int l = 0; l < c_p.n_scalar; ++l) z.sv[l * z.sz + go] = z.sv[l * z.sz + g];
-      if (c_p.sst) z.mut[go] = z.mut[g];
-    }
+    PointState<NS> s;
+    load_point<NS>(z, g, s);
+    extrapolate_point<NS>(z, g, step, 1, s, 0);
   } else {
     const double r_pos = u_face + 2 * a_b / (gamma_b - 1);
     const double u_inf = b.u * nx + b.v * ny + b.w * nz;
@@ -717,15 +780,10 @@ __device__ __forceinline__ void bc_farfield_point(const DevZone &z, const BcFace
 template <int NS>
 __device__ __forceinline__ void bc_back_pressure_point(const DevZone &z, const BcFace &b, int with_cv, int i, int j, int k) {
   const int g = gidx(z, i, j, k);
-  for (int gg = 1; gg <= z.ngg; ++gg) {
-    const int go = g + gg * b.dir_stride;
-    for (int l = 0; l < 4; ++l) z.bv[l * z.sz + go] = z.bv[l * z.sz + g];
-    z.bv[4 * z.sz + go] = b.pressure;
-    z.bv[5 * z.sz + go] = z.bv[5 * z.sz + g];
-    for (int l = 0; l < c_p.n_scalar; ++l) z.sv[l * z.sz + go] = z.sv[l * z.sz + g];
-    if (c_p.sst) z.mut[go] = z.mut[g];
-    if (with_cv) cv_from_bv_point<NS>(z, go);
-  }
+  PointState<NS> s;
+  load_point<NS>(z, g, s);
+  s.b[4] = b.pressure;
+  extrapolate_point<NS>(z, g, b.dir_stride, 1, s, with_cv);
 }
 
 // subsonic inflow from total conditions, air (BoundCond.cuh:528-634)
@@ -785,8 +843,10 @@ template <int NS>
 OSTC_BC_KERNEL(bc_outflow_kernel, bc_outflow_point<NS>)
 template <int NS>
 OSTC_BC_KERNEL(bc_inflow_kernel, bc_inflow_point<NS>)
-static OSTC_BC_KERNEL(bc_symmetry_kernel, bc_symmetry_point)
-static OSTC_BC_KERNEL(bc_periodic_kernel, bc_periodic_point)
+template <int NS>
+OSTC_BC_KERNEL(bc_symmetry_kernel, bc_symmetry_point<NS>)
+template <int NS>
+OSTC_BC_KERNEL(bc_periodic_kernel, bc_periodic_point<NS>)
 template <int NS>
 OSTC_BC_KERNEL(bc_wall_kernel, bc_wall_point<NS>)
 template <int NS>
@@ -803,12 +863,12 @@ __device__ __forceinline__ void bc_point(const DevZone &z, const BcFace &b, int 
   switch (b.type) {
     case OSTC_BC_OUTFLOW: bc_outflow_point<NS>(z, b, with_cv, i, j, k); break;
     case OSTC_BC_INFLOW: bc_inflow_point<NS>(z, b, with_cv, i, j, k); break;
-    case OSTC_BC_SYMMETRY: bc_symmetry_point(z, b, with_cv, i, j, k); break;
+    case OSTC_BC_SYMMETRY: bc_symmetry_point<NS>(z, b, with_cv, i, j, k); break;
     case OSTC_BC_WALL: bc_wall_point<NS>(z, b, with_cv, i, j, k); break;
     case OSTC_BC_FARFIELD: bc_farfield_point<NS>(z, b, with_cv, i, j, k); break;
     case OSTC_BC_BACK_PRESSURE: bc_back_pressure_point<NS>(z, b, with_cv, i, j, k); break;
     case OSTC_BC_SUBSONIC_INFLOW: bc_subsonic_inflow_point(z, b, with_cv, i, j, k); break;
-    case OSTC_BC_PERIODIC: bc_periodic_point(z, b, with_cv, i, j, k); break;
+    case OSTC_BC_PERIODIC: bc_periodic_point<NS>(z, b, with_cv, i, j, k); break;
     default: break;
   }
 }
@@ -830,26 +890,22 @@ __device__ __forceinline__ void interface_point(const DevZone &z, const DevZone 
   const int g = gidx(z, idx[0], idx[1], idx[2]);
   const int gt = gidx(t, it[0], it[1], it[2]);
   const int plane = f.direction > 0 ? f.rs[f.face] : f.rs[f.face] + f.ld[f.face] * (f.np[f.face] - 1);
+  PointState<NS> s;
+  load_point<NS>(t, gt, s);
   if (idx[f.face] == plane) {
-    for (int l = 0; l < 6; ++l) {
-      const double ave = 0.5 * (t.bv[l * t.sz + gt] + z.bv[l * z.sz + g]);
-      z.bv[l * z.sz + g] = ave;
-      t.bv[l * t.sz + gt] = ave;
-    }
-    for (int l = 0; l < c_p.n_scalar; ++l) {
-      const double ave = 0.5 * (t.sv[l * t.sz + gt] + z.sv[l * z.sz + g]);
-      z.sv[l * z.sz + g] = ave;
-      t.sv[l * t.sz + gt] = ave;
-    }
-    const double u = z.bv[z.sz + g], v = z.bv[2 * z.sz + g], w = z.bv[3 * z.sz + g];
-    const double vel = sqrt(u * u + v * v + w * w);
+    PointState<NS> o;
+    load_point<NS>(z, g, o);
+#pragma unroll
+    for (int l = 0; l < 6; ++l) s.b[l] = 0.5 * (s.b[l] + o.b[l]);
+#pragma unroll
+    for (int l = 0; l < NS + 2; ++l) s.y[l] = 0.5 * (s.y[l] + o.y[l]);
+    store_point<NS>(t, gt, s, false);
+    const double vel = sqrt(s.b[1] * s.b[1] + s.b[2] * s.b[2] + s.b[3] * s.b[3]);
     z.vel[g] = vel;
     t.vel[gt] = vel;
-  } else {
-    for (int l = 0; l < 6; ++l) z.bv[l * z.sz + g] = t.bv[l * t.sz + gt];
-    for (int l = 0; l < c_p.n_scalar; ++l) z.sv[l * z.sz + g] = t.sv[l * t.sz + gt];
   }
-  if (with_cv) cv_from_bv_point<NS>(z, g);
+  store_point<NS>(z, g, s, false);
+  if (with_cv) store_cv<NS>(z, g, s);
 }
 
 template <int NS>
@@ -1238,8 +1294,8 @@ cudaError_t launch_bc(const DevZone &z, const BcFace &b, int with_cv, cudaStream
   switch (b.type) {
     case OSTC_BC_OUTFLOW: bc_outflow_kernel<NS><<<grid, blk, 0, s>>>(z, b, with_cv); break;
     case OSTC_BC_INFLOW: bc_inflow_kernel<NS><<<grid, blk, 0, s>>>(z, b, with_cv); break;
-    case OSTC_BC_SYMMETRY: bc_symmetry_kernel<<<grid, blk, 0, s>>>(z, b, with_cv); break;
-    case OSTC_BC_PERIODIC: bc_periodic_kernel<<<grid, blk, 0, s>>>(z, b, with_cv); break;
+    case OSTC_BC_SYMMETRY: bc_symmetry_kernel<NS><<<grid, blk, 0, s>>>(z, b, with_cv); break;
+    case OSTC_BC_PERIODIC: bc_periodic_kernel<NS><<<grid, blk, 0, s>>>(z, b, with_cv); break;
     case OSTC_BC_WALL: bc_wall_kernel<NS><<<grid, blk, 0, s>>>(z, b, with_cv); break;
     case OSTC_BC_FARFIELD: bc_farfield_kernel<NS><<<grid, blk, 0, s>>>(z, b, with_cv); break;
     case OSTC_BC_BACK_PRESSURE: bc_back_pressure_kernel<NS><<<grid, blk, 0, s>>>(z, b, with_cv); break;
