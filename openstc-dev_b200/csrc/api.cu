@@ -121,8 +121,8 @@ ostc_status ensure_param(ostc_ctx *ctx, cudaStream_t s) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     CK(cudaStreamIsCapturing(s, &cap));
     if (cap != cudaStreamCaptureStatusNone) return fail(ctx, OSTC_ERR_INVALID_ARG);
-    CK(upload_param(ctx->dp, s));
-    if (ctx->batched || ctx->face_batched) CK(upload_zones(ctx->dz.data(), (int)ctx->dz.size(), s));
+    CK(upload_param(ctx->dp, ctx->ns, ctx->nt, s));
+    if (ctx->batched || ctx->face_batched) CK(upload_zones(ctx->dz.data(), (int)ctx->dz.size(), ctx->ns, ctx->nt, s));
     g_uploaded = ctx;
   }
   return OSTC_OK;
@@ -1172,7 +1172,7 @@ ostc_status ostc_set_interfaces(ostc_ctx *ctx, const ostc_interface *f, int n) {
 ostc_status ostc_eliminate_k_gradient(ostc_ctx *ctx, int with_cv, void *stream) {
   if (!ctx) return OSTC_ERR_INVALID_ARG;
   if (ensure_param(ctx, S(stream))) return ctx->last;
-  for (auto &z : ctx->dz) CK(launch_eliminate_k(z, with_cv, S(stream)));
+  for (auto &z : ctx->dz) CK(launch_eliminate_k(z, ctx->dp.n_scalar, with_cv ? ctx->dp.n_var : 0, S(stream)));
   return OSTC_OK;
 }
 

@@ -1124,6 +1124,9 @@ template <int NS>
 struct CvOp {
   __device__ void operator()(const DevZone &z, int bx, int by, int bz) const { cv_from_bv_cells<NS>(z, bx, by, bz); }
 };
+// (every Op carries its species count: a kernel of the same name in two units would be
+// one symbol, and run with either unit's zone table)
+template <int NS>
 struct VelocityOp {
   __device__ void operator()(const DevZone &z, int bx, int by, int bz) const { velocity_cells(z, bx, by, bz); }
 };
@@ -1132,6 +1135,7 @@ struct DtOp {
   unsigned long long *dt_bits;
   __device__ void operator()(const DevZone &z, int bx, int by, int bz) const { dt_cells<NS>(z, bx, by, bz, dt_bits); }
 };
+template <int NS>
 struct StoreLastOp {
   __device__ void operator()(const DevZone &z, int bx, int by, int bz) const { store_last_cells(z, bx, by, bz); }
 };
@@ -1172,22 +1176,30 @@ cudaError_t launch_table(const CellTable &tab, const Op &op, cudaStream_t s) {
 }  // namespace
 
 #ifndef OSTC_NS_UNIT
-cudaError_t upload_zones(const DevZone *z, int n, cudaStream_t s) {
+// the kernel units a context of ns species and nt turbulence scalars launches, besides
+// this one: its sweeps' and, for counts other than 0 and 9, its per-cell kernels'
+struct UnitUploads {
+  cudaError_t (*param[2])(const DevParam &, cudaStream_t);
+  cudaError_t (*zones[2])(const DevZone *, int, cudaStream_t);
+};
+static UnitUploads unit_uploads(int ns, int nt) {
+  if (nt > 0)
+    return ns == 9 ? UnitUploads{{upload_param_flux9t}, {upload_zones_flux9t}}
+                   : UnitUploads{{upload_param_flux0t}, {upload_zones_flux0t}};
+  if (ns == 0) return {{upload_param_flux0}, {upload_zones_flux0}};
+  if (ns == 9) return {{upload_param_flux9}, {upload_zones_flux9}};
+  if (ns <= 5) return {{upload_param_flux_ns_a, upload_param_ns_a}, {upload_zones_flux_ns_a, upload_zones_ns_a}};
+  if (ns <= 10) return {{upload_param_flux_ns_b, upload_param_ns_b}, {upload_zones_flux_ns_b, upload_zones_ns_b}};
+  if (ns <= 15) return {{upload_param_flux_ns_c, upload_param_ns_c}, {upload_zones_flux_ns_c, upload_zones_ns_c}};
+  return {{upload_param_flux_ns_d, upload_param_ns_d}, {upload_zones_flux_ns_d, upload_zones_ns_d}};
+}
+
+cudaError_t upload_zones(const DevZone *z, int n, int ns, int nt, cudaStream_t s) {
   if (n < 0 || n > kMaxTableZones) return cudaErrorInvalidValue;
   cudaError_t e = n ? cudaMemcpyToSymbolAsync(c_zones, z, sizeof(DevZone) * n, 0, cudaMemcpyHostToDevice, s)
                     : cudaSuccess;
-  if (e == cudaSuccess) e = upload_zones_flux0(z, n, s);
-  if (e == cudaSuccess) e = upload_zones_flux9(z, n, s);
-  if (e == cudaSuccess) e = upload_zones_flux0t(z, n, s);
-  if (e == cudaSuccess) e = upload_zones_flux9t(z, n, s);
-  if (e == cudaSuccess) e = upload_zones_ns_a(z, n, s);
-  if (e == cudaSuccess) e = upload_zones_flux_ns_a(z, n, s);
-  if (e == cudaSuccess) e = upload_zones_ns_b(z, n, s);
-  if (e == cudaSuccess) e = upload_zones_flux_ns_b(z, n, s);
-  if (e == cudaSuccess) e = upload_zones_ns_c(z, n, s);
-  if (e == cudaSuccess) e = upload_zones_flux_ns_c(z, n, s);
-  if (e == cudaSuccess) e = upload_zones_ns_d(z, n, s);
-  if (e == cudaSuccess) e = upload_zones_flux_ns_d(z, n, s);
+  for (auto f : unit_uploads(ns, nt).zones)
+    if (f && e == cudaSuccess) e = f(z, n, s);
   return e;
 }
 #endif  // OSTC_NS_UNIT
@@ -1200,9 +1212,9 @@ cudaError_t launch_cells_table(CellOp op, const CellTable &tab, const CellArgs &
     case CellOp::UpdateRK: return launch_table(tab, UpdateOp<NS>{a.dt, a.dt_dev, a.rk}, s);
     case CellOp::Properties: return launch_table(tab, PropertiesOp<NS>{}, s);
     case CellOp::CvFromBv: return launch_table(tab, CvOp<NS>{}, s);
-    case CellOp::Velocity: return launch_table(tab, VelocityOp{}, s);
+    case CellOp::Velocity: return launch_table(tab, VelocityOp<NS>{}, s);
     case CellOp::Dt: return launch_table(tab, DtOp<NS>{a.dt_bits}, s);
-    case CellOp::StoreLast: return launch_table(tab, StoreLastOp{}, s);
+    case CellOp::StoreLast: return launch_table(tab, StoreLastOp<NS>{}, s);
     case CellOp::InitMut: return launch_table(tab, InitMutOp<NS>{}, s);
     default: return cudaErrorInvalidValue;
   }
@@ -1261,27 +1273,24 @@ cudaError_t launch_residual_final(const double *partial, int n_part, double n_to
 // Every ghost plane k = +-1 .. +-ngg of bv, sv (and cv) becomes a copy of the
 // plane k = 0, over the whole ghosted (i, j) range, so every difference
 // across k vanishes.
-static __global__ void eliminate_k_kernel(DevZone z, int with_cv) {
+// One variable per thread (blockIdx.z), read once and written to the 2 ngg planes.
+static __global__ void eliminate_k_kernel(DevZone z) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x - z.ngg;
   const int j = blockIdx.y * blockDim.y + threadIdx.y - z.ngg;
   if (i >= z.mx + z.ngg || j >= z.my + z.ngg) return;
-  const int g0 = gidx(z, i, j, 0);
-  const long long S = z.sz;
-  for (int k = 1; k <= z.ngg; ++k) {
-    const int gp = g0 + k * z.d1, gm = g0 - k * z.d1;
-    for (int l = 0; l < 6; ++l) z.bv[l * S + gp] = z.bv[l * S + gm] = z.bv[l * S + g0];
-    for (int l = 0; l < c_p.n_scalar; ++l) z.sv[l * S + gp] = z.sv[l * S + gm] = z.sv[l * S + g0];
-    if (with_cv)
-      for (int l = 0; l < c_p.n_var; ++l) z.cv[l * S + gp] = z.cv[l * S + gm] = z.cv[l * S + g0];
-  }
+  const int v = blockIdx.z;  // bv, then sv, then cv
+  double *q = v < 6 ? z.bv + v * z.sz : (v < 6 + c_p.n_scalar ? z.sv + (v - 6) * z.sz : z.cv + (v - 6 - c_p.n_scalar) * z.sz);
+  q += gidx(z, i, j, 0);
+  const double x = *q;
+  for (int k = 1; k <= z.ngg; ++k) q[k * z.d1] = q[-k * z.d1] = x;
 }
 
 #ifndef OSTC_NS_UNIT
-cudaError_t launch_eliminate_k(const DevZone &z, int with_cv, cudaStream_t s) {
+cudaError_t launch_eliminate_k(const DevZone &z, int n_scalar, int n_cv, cudaStream_t s) {
   if (z.mz != 1) return cudaSuccess;
   const dim3 blk(32, 8);
-  const dim3 grid((z.mx + 2 * z.ngg + 31) / 32, (z.my + 2 * z.ngg + 7) / 8);
-  eliminate_k_kernel<<<grid, blk, 0, s>>>(z, with_cv);
+  const dim3 grid((z.mx + 2 * z.ngg + 31) / 32, (z.my + 2 * z.ngg + 7) / 8, 6 + n_scalar + n_cv);
+  eliminate_k_kernel<<<grid, blk, 0, s>>>(z);
   return cudaGetLastError();
 }
 #endif  // OSTC_NS_UNIT
@@ -1477,21 +1486,13 @@ cudaError_t stage_timeouts(int *any) {
   return cudaSuccess;
 }
 
-// this unit's parameters and those of the flux units (flux0.cu, flux9.cu)
-cudaError_t upload_param(const DevParam &p, cudaStream_t s) {
+// this unit's parameters and those of the units that ns species and nt turbulence
+// scalars launch: switching between contexts costs two or three copies (13 units: 60 us
+// of a 94 us residual of a small block, when several contexts take turns)
+cudaError_t upload_param(const DevParam &p, int ns, int nt, cudaStream_t s) {
   cudaError_t e = cudaMemcpyToSymbolAsync(c_p, &p, sizeof(DevParam), 0, cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = upload_param_flux0(p, s);
-  if (e == cudaSuccess) e = upload_param_flux9(p, s);
-  if (e == cudaSuccess) e = upload_param_flux0t(p, s);
-  if (e == cudaSuccess) e = upload_param_flux9t(p, s);
-  if (e == cudaSuccess) e = upload_param_ns_a(p, s);
-  if (e == cudaSuccess) e = upload_param_flux_ns_a(p, s);
-  if (e == cudaSuccess) e = upload_param_ns_b(p, s);
-  if (e == cudaSuccess) e = upload_param_flux_ns_b(p, s);
-  if (e == cudaSuccess) e = upload_param_ns_c(p, s);
-  if (e == cudaSuccess) e = upload_param_flux_ns_c(p, s);
-  if (e == cudaSuccess) e = upload_param_ns_d(p, s);
-  if (e == cudaSuccess) e = upload_param_flux_ns_d(p, s);
+  for (auto f : unit_uploads(ns, nt).param)
+    if (f && e == cudaSuccess) e = f(p, s);
   return e;
 }
 #endif  // OSTC_NS_UNIT

@@ -120,8 +120,8 @@ cudaError_t launch_cells(CellOp op, const DevZone &z, const CellArgs &a, cudaStr
 // CvFromBv, Velocity
 template <int NS>
 cudaError_t launch_cells_table(CellOp op, const CellTable &tab, const CellArgs &a, cudaStream_t s);
-// the zone tables of every kernel unit
-cudaError_t upload_zones(const DevZone *z, int n, cudaStream_t s);
+// the zone tables of the kernel units of ns species and nt turbulence scalars
+cudaError_t upload_zones(const DevZone *z, int n, int ns, int nt, cudaStream_t s);
 cudaError_t upload_zones_flux0(const DevZone *z, int n, cudaStream_t s);   // flux0.cu
 cudaError_t upload_zones_flux9(const DevZone *z, int n, cudaStream_t s);   // flux9.cu
 cudaError_t upload_zones_flux0t(const DevZone *z, int n, cudaStream_t s);  // flux0t.cu
@@ -202,8 +202,9 @@ cudaError_t launch_monitor_advance(int *counter, cudaStream_t s);
 cudaError_t launch_statistics(const DevZone &z, const int *step, int start, const StatSums &st, int ns,
                               cudaStream_t s);
 // 2-D blocks: copy the plane k = 0 into every k ghost plane (no-op when mz > 1)
-cudaError_t launch_eliminate_k(const DevZone &z, int with_cv, cudaStream_t s);
-cudaError_t upload_param(const DevParam &p, cudaStream_t s);
+// (bv, n_scalar planes of sv, n_cv planes of cv)
+cudaError_t launch_eliminate_k(const DevZone &z, int n_scalar, int n_cv, cudaStream_t s);
+cudaError_t upload_param(const DevParam &p, int ns, int nt, cudaStream_t s);
 cudaError_t upload_param_flux0(const DevParam &p, cudaStream_t s);   // flux0.cu
 cudaError_t upload_param_flux9(const DevParam &p, cudaStream_t s);   // flux9.cu
 cudaError_t upload_param_flux0t(const DevParam &p, cudaStream_t s);  // flux0t.cu
