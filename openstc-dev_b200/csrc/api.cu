@@ -80,8 +80,8 @@ struct ostc_ctx {
   std::vector<StatSums> stats;
   // steady path: spectral radii (3 interior planes), DPLUR buffers (dq layout),
   // DPLUR point-implicit chemistry (LU factors + pivots, or DA divisors)
-  std::vector<double *> isr, dq0, dqk, lu, da;
-  std::vector<unsigned char *> piv;
+  std::vector<double *> isr;
+  CellTable wall_tab;  // tiles of the wall faces (DPLUR clears its iterate there)
   std::vector<void *> owned;  // allocations of this context to free
   // split chemistry (chem_mode 1, 2): SoA staging of the largest block and totals
   ostc_surrogate *sur = nullptr;
@@ -333,6 +333,15 @@ ostc_status build_tables(ostc_ctx *ctx) {
     if (!ctx->ifaces.empty())
       CK(cudaMemcpy(ctx->ifaces_dev, ctx->ifaces.data(), sizeof(Iface) * ctx->ifaces.size(), cudaMemcpyHostToDevice));
   }
+  // the wall faces DPLUR clears its iterate on
+  const size_t wall0 = all.size();
+  for (size_t q = 0; q < ctx->faces.size(); ++q) {
+    const BcFace &b = ctx->faces[q];
+    if (b.type != OSTC_BC_WALL) continue;
+    const int n[3] = {b.re[0] - b.rs[0] + 1, b.re[1] - b.rs[1] + 1, b.re[2] - b.rs[2] + 1};
+    wave_tiles((int)q, b.face, n);
+  }
+  const size_t wall1 = all.size();
   if (!ctx->faces.empty() && !ctx->faces_dev) {
     CK(cudaMalloc(&ctx->faces_dev, sizeof(BcFace) * ctx->faces.size()));
     CK(cudaMemcpy(ctx->faces_dev, ctx->faces.data(), sizeof(BcFace) * ctx->faces.size(), cudaMemcpyHostToDevice));
@@ -353,6 +362,8 @@ ostc_status build_tables(ostc_ctx *ctx) {
     return t;
   };
   for (int c = 0; c < 3; ++c) ctx->cell_tab[c] = table(c);
+  ctx->wall_tab.tiles = ctx->tab_dev + wall0;
+  ctx->wall_tab.n = (int)(wall1 - wall0);
   for (int d = 0; d < 3; ++d)
     for (int v = 0; v < 2; ++v) {
       ctx->flux_tab[d][v] = table(3 + 2 * d + v);
@@ -451,6 +462,39 @@ ostc_status cells_all(ostc_ctx *ctx, CellOp op, int table, const CellArgs &a, cu
   return OSTC_OK;
 }
 
+// one steady kernel family over every zone: a tile-table launch when batched, else one
+// launch per zone
+ostc_status steady_all(ostc_ctx *ctx, SteadyOp op, const SteadyArgs &a, cudaStream_t s) {
+  if (ctx->batched) {
+    CK(dispatch_ns(ctx->ns, [&](auto n) {
+      return launch_steady_table<decltype(n)::value>(op, ctx->cell_tab[0], a, s);
+    }));
+    return OSTC_OK;
+  }
+  for (auto &z : ctx->dz)
+    CK(dispatch_ns(ctx->ns, [&](auto n) { return launch_steady<decltype(n)::value>(op, z, a, nullptr, s); }));
+  return OSTC_OK;
+}
+
+// the residual partials and the state check of every zone
+ostc_status residual_all(ostc_ctx *ctx, cudaStream_t s) {
+  CellArgs a;
+  a.n_part = ctx->n_part_per_zone;
+  a.bad = ctx->bad_key;
+  a.step = ctx->hist_counter;
+  a.partial = ctx->res_partial;
+  if (ctx->batched) {
+    CK(launch_residual_table((int)ctx->dz.size(), a, s));
+    return OSTC_OK;
+  }
+  for (size_t b = 0; b < ctx->dz.size(); ++b) {
+    a.partial = ctx->res_partial + 4 * ctx->n_part_per_zone * b;
+    a.block = (int)b;
+    CK(launch_cells<0>(CellOp::ResidualPartial, ctx->dz[b], a, s));
+  }
+  return OSTC_OK;
+}
+
 // repack the reference's 80-byte gxl::Matrix<real,3,3,1> records into 9 planes
 __global__ void repack_metric_kernel(const unsigned char *src, double *dst, long long n) {
   const long long q = blockIdx.x * 256ll + threadIdx.x;
@@ -460,21 +504,34 @@ __global__ void repack_metric_kernel(const unsigned char *src, double *dst, long
   for (int c = 0; c < 9; ++c) dst[c * n + q] = m[c];
 }
 
-__global__ void step_end_kernel(const double *partial, int n_part, double n_total, const double *dt_dev,
-                                double dt_fixed, double *hist_res, double *hist_dt, int *counter, int cap) {
-  if (threadIdx.x != 0) return;
-  const int s = *counter;
-  if (s < cap) {
-    if (hist_res && partial) {
-      for (int l = 0; l < 4; ++l) {
-        double acc = 0;
-        for (int p = 0; p < n_part; ++p) acc += partial[p * 4 + l];
-        hist_res[s * 4 + l] = sqrt(acc / n_total);
-      }
+// one CTA of 256 threads: the partials summed in a fixed order (each thread its strided
+// share, then a tree), 8 us for the 2664 partials of 9 blocks against 222 by one thread
+__global__ void __launch_bounds__(256) step_end_kernel(const double *partial, int n_part, double n_total,
+                                                       const double *dt_dev, double dt_fixed, double *hist_res,
+                                                       double *hist_dt, int *counter, int cap) {
+  __shared__ double red[4][256];
+  const int s = *counter, t = threadIdx.x;
+  if (s < cap && hist_res && partial) {
+    double acc[4] = {0, 0, 0, 0};
+    for (int p = t; p < n_part; p += 256)
+#pragma unroll
+      for (int l = 0; l < 4; ++l) acc[l] += partial[p * 4 + l];
+#pragma unroll
+    for (int l = 0; l < 4; ++l) red[l][t] = acc[l];
+    __syncthreads();
+    for (int o = 128; o > 0; o >>= 1) {
+      if (t < o)
+#pragma unroll
+        for (int l = 0; l < 4; ++l) red[l][t] += red[l][t + o];
+      __syncthreads();
     }
-    if (hist_dt) hist_dt[s] = dt_dev ? *dt_dev : dt_fixed;
+    if (t < 4) hist_res[s * 4 + t] = sqrt(red[t][0] / n_total);
   }
-  *counter = s + 1;
+  __syncthreads();  // every thread has read the counter
+  if (t == 0) {
+    if (s < cap && hist_dt) hist_dt[s] = dt_dev ? *dt_dev : dt_fixed;
+    *counter = s + 1;
+  }
 }
 
 void fill_devzone(const ostc_zone &z, DevZone &d) {
@@ -512,7 +569,8 @@ void fill_devzone(const ostc_zone &z, DevZone &d) {
   d.wall = z.wall_distance;
   d.dt_local = z.dt_local;
   d.bv_last = z.bv_last;
-  d.isr = nullptr;
+  d.isr = d.dq0 = d.dqk = d.lu = d.da = nullptr;
+  d.piv = nullptr;
   d.tsj = z.turb_src_jac;
   d.jac = z.jac;
 }
@@ -909,11 +967,11 @@ ostc_status ostc_create(const ostc_config *cfg, const ostc_param *param, const o
           if (!da) return fail(ctx, OSTC_ERR_CUDA, cudaErrorMemoryAllocation);
         }
       }
-      c->dq0.push_back(d0);
-      c->dqk.push_back(dk);
-      c->lu.push_back(lu);
-      c->piv.push_back(pv);
-      c->da.push_back(da);
+      z.dq0 = d0;
+      z.dqk = dk;
+      z.lu = lu;
+      z.piv = pv;
+      z.da = da;
     }
   }
   if (cfg->chem_mode != 0) {
@@ -1262,16 +1320,8 @@ static ostc_status enqueue_step(ostc_ctx *ctx, bool with_hist, cudaStream_t s) {
     if ((st = ostc_update_physical_properties(ctx, s))) return st;
   }
   if (with_hist) {
-    CellArgs a;
-    a.n_part = ctx->n_part_per_zone;
-    a.bad = ctx->bad_key;
-    a.step = ctx->hist_counter;
-    for (size_t b = 0; b < ctx->dz.size(); ++b) {
-      a.partial = ctx->res_partial + 4 * ctx->n_part_per_zone * b;
-      a.block = (int)b;
-      CK(launch_cells<0>(CellOp::ResidualPartial, ctx->dz[b], a, s));
-    }
-    step_end_kernel<<<1, 32, 0, s>>>(ctx->res_partial, ctx->n_part_per_zone * (int)ctx->dz.size(), ctx->n_total,
+    if ((st = residual_all(ctx, s))) return st;
+    step_end_kernel<<<1, 256, 0, s>>>(ctx->res_partial, ctx->n_part_per_zone * (int)ctx->dz.size(), ctx->n_total,
                                      ctx->cfg.fixed_time_step ? nullptr : (const double *)ctx->dt_bits, ctx->cfg.dt,
                                      ctx->hist_res, ctx->hist_dt, ctx->hist_counter, ctx->hist_cap);
     CK(cudaGetLastError());
@@ -1409,70 +1459,53 @@ ostc_status ostc_local_time_step(ostc_ctx *ctx, void *stream) {
   CellArgs a;
   a.dt_bits = ctx->dt_bits;
   CK(launch_cells<0>(CellOp::DtReset, ctx->dz[0], a, S(stream)));
-  for (auto &z : ctx->dz)
-    CK(dispatch_ns(ctx->ns, [&](auto n) { return launch_cells<decltype(n)::value>(CellOp::Dt, z, a, S(stream)); }));
-  return OSTC_OK;
+  return cells_all(ctx, CellOp::Dt, 0, a, S(stream));
 }
 
 ostc_status ostc_implicit_treatment(ostc_ctx *ctx, void *stream) {
   if (!ctx || !ctx->cfg.steady) return OSTC_ERR_INVALID_ARG;
   if (ensure_param(ctx, S(stream))) return ctx->last;
   cudaStream_t s = S(stream);
+  ostc_status st;
+  SteadyArgs a;
+  a.spec = ctx->spec_mech;
   if (ctx->cfg.implicit_method == 0) {
     // ImplicitTreatmentHPP.cuh:11-48: the chemistry's EPI / DA, then SST's point-implicit k, omega sources
-    if (ctx->has_source && ctx->prm.chemSrcMethod != 0)
-      for (auto &z : ctx->dz)
-        CK(dispatch_ns(ctx->ns, [&](auto n) {
-          return launch_steady<decltype(n)::value>(SteadyOp::ChemImplicit, z, SteadyArgs{}, nullptr, s);
-        }));
-    if (ctx->dp.sst && ctx->dp.turb_implicit == 1)
-      for (auto &z : ctx->dz) CK(launch_steady<0>(SteadyOp::TurbImplicit, z, SteadyArgs{}, nullptr, s));
+    if (ctx->has_source && ctx->prm.chemSrcMethod != 0 && (st = steady_all(ctx, SteadyOp::ChemImplicit, a, s))) return st;
+    if (ctx->dp.sst && ctx->dp.turb_implicit == 1 && (st = steady_all(ctx, SteadyOp::TurbImplicit, a, s))) return st;
     return OSTC_OK;
   }
   // DPLUR (DPLUR.cuh:283-312): no exchange between blocks inside the sweeps (quirk A11)
-  for (size_t b = 0; b < ctx->dz.size(); ++b) {
-    const DevZone &z = ctx->dz[b];
-    SteadyArgs a;
-    a.dq0 = ctx->dq0[b];
-    a.lu = ctx->lu[b];
-    a.piv = ctx->piv[b];
-    a.da = ctx->da[b];
-    CK(dispatch_ns(ctx->ns, [&](auto n) { return launch_steady<decltype(n)::value>(SteadyOp::DplurDq0, z, a, nullptr, s); }));
-    double *cur = z.dq, *nxt = ctx->dqk[b];
-    for (int it = 0; it < ctx->cfg.DPLUR_inner_step; ++it) {
+  const int n = ctx->cfg.DPLUR_inner_step;
+  a.buf = n > 0 ? n & 1 : 0;
+  if ((st = steady_all(ctx, SteadyOp::DplurDq0, a, s))) return st;
+  for (int it = 0; it < n; ++it) {
+    if (ctx->batched) {
+      CK(launch_wall_zero_table(ctx->wall_tab, ctx->faces_dev, a.buf, s));
+    } else {
       for (size_t q = 0; q < ctx->faces.size(); ++q) {
-        if (ctx->face_zone[q] != (int)b || ctx->faces[q].type != OSTC_BC_WALL) continue;
-        SteadyArgs w;
-        w.dq_out = cur;
-        CK(dispatch_ns(ctx->ns, [&](auto n) {
-          return launch_steady<decltype(n)::value>(SteadyOp::WallDqZero, z, w, &ctx->faces[q], s);
+        if (ctx->faces[q].type != OSTC_BC_WALL) continue;
+        CK(dispatch_ns(ctx->ns, [&](auto m) {
+          return launch_steady<decltype(m)::value>(SteadyOp::WallDqZero, ctx->dz[ctx->face_zone[q]], a, &ctx->faces[q], s);
         }));
       }
-      a.dq_in = cur;
-      a.dq_out = nxt;
-      CK(dispatch_ns(ctx->ns, [&](auto n) { return launch_steady<decltype(n)::value>(SteadyOp::DplurSweep, z, a, nullptr, s); }));
-      std::swap(cur, nxt);
     }
-    a.dq_in = cur;
-    CK(dispatch_ns(ctx->ns, [&](auto n) { return launch_steady<decltype(n)::value>(SteadyOp::DplurFinish, z, a, nullptr, s); }));
+    a.final_div = it + 1 == n;
+    if ((st = steady_all(ctx, SteadyOp::DplurSweep, a, s))) return st;
+    a.buf ^= 1;
   }
-  return OSTC_OK;
+  return n > 0 ? OSTC_OK : steady_all(ctx, SteadyOp::DplurFinish, a, s);
 }
 
 ostc_status ostc_update_bv(ostc_ctx *ctx, void *stream) {
   if (!ctx || !ctx->cfg.steady) return OSTC_ERR_INVALID_ARG;
   if (ensure_param(ctx, S(stream))) return ctx->last;
-  for (auto &z : ctx->dz)
-    CK(dispatch_ns(ctx->ns, [&](auto n) {
-      return launch_steady<decltype(n)::value>(SteadyOp::UpdateBv, z, SteadyArgs{}, nullptr, S(stream));
-    }));
-  return OSTC_OK;
+  return steady_all(ctx, SteadyOp::UpdateBv, {}, S(stream));
 }
 
 static ostc_status enqueue_steady_step(ostc_ctx *ctx, bool with_hist, cudaStream_t s) {
   ostc_status st;
-  if (with_hist)
-    for (auto &z : ctx->dz) CK(launch_cells<0>(CellOp::StoreLast, z, {}, s));
+  if (with_hist && (st = cells_all(ctx, CellOp::StoreLast, 0, {}, s))) return st;
   if ((st = ostc_compute_rhs(ctx, s))) return st;
   if ((st = ostc_local_time_step(ctx, s))) return st;
   if ((st = ostc_implicit_treatment(ctx, s))) return st;
@@ -1482,16 +1515,8 @@ static ostc_status enqueue_steady_step(ostc_ctx *ctx, bool with_hist, cudaStream
   if ((st = ostc_eliminate_k_gradient(ctx, 0, s))) return st;  // 2-D only (SteadySim.cuh:101-107)
   if ((st = ostc_update_physical_properties(ctx, s))) return st;
   if (with_hist) {
-    CellArgs a;
-    a.n_part = ctx->n_part_per_zone;
-    a.bad = ctx->bad_key;
-    a.step = ctx->hist_counter;
-    for (size_t b = 0; b < ctx->dz.size(); ++b) {
-      a.partial = ctx->res_partial + 4 * ctx->n_part_per_zone * b;
-      a.block = (int)b;
-      CK(launch_cells<0>(CellOp::ResidualPartial, ctx->dz[b], a, s));
-    }
-    step_end_kernel<<<1, 32, 0, s>>>(ctx->res_partial, ctx->n_part_per_zone * (int)ctx->dz.size(), ctx->n_total,
+    if ((st = residual_all(ctx, s))) return st;
+    step_end_kernel<<<1, 256, 0, s>>>(ctx->res_partial, ctx->n_part_per_zone * (int)ctx->dz.size(), ctx->n_total,
                                      nullptr, 0.0, ctx->hist_res, nullptr, ctx->hist_counter, ctx->hist_cap);
     CK(cudaGetLastError());
   }

@@ -171,17 +171,26 @@ __device__ __forceinline__ void chemistry_jacobian(double rho, const double *Y, 
                                                    double *J) {
   const int nr = c_p.n_reac;
 #pragma unroll 1
-  for (int m = 0; m < NS; ++m) {
+  for (int e = 0; e < NS * NS; ++e) J[e] = 0;
+  // each reaction adds to the entries of its own species only
+#pragma unroll 1
+  for (int r = 0; r < nr; ++r)
 #pragma unroll 1
     for (int n = 0; n < NS; ++n) {
-      double zz = 0;
-      if (Y[n] > 1e-25) {
-        for (int r = 0; r < nr; ++r)
-          zz += (c_p.nub[r][m] - c_p.nuf[r][m]) * (c_p.nuf[r][n] * q1[r] - c_p.nub[r][n] * q2[r]);
-        zz /= rho * Y[n];
+      const int nf = c_p.nuf[r][n], nb = c_p.nub[r][n];
+      if (!(nf | nb)) continue;
+      const double d = nf * q1[r] - nb * q2[r];
+#pragma unroll 1
+      for (int m = 0; m < NS; ++m) {
+        const int net = c_p.nub[r][m] - c_p.nuf[r][m];
+        if (net) J[m * NS + n] += net * d;
       }
-      J[m * NS + n] = c_p.mw[m] * zz * 1e+3;
     }
+#pragma unroll 1
+  for (int n = 0; n < NS; ++n) {
+    const double s = Y[n] > 1e-25 ? 1.0 / (rho * Y[n]) : 0.0;
+#pragma unroll 1
+    for (int m = 0; m < NS; ++m) J[m * NS + n] = c_p.mw[m] * (J[m * NS + n] * s) * 1e+3;
   }
 }
 

@@ -80,6 +80,11 @@ struct DevZone {
   // staged flux kernels copy starts on a 16-byte boundary, so that their tile
   // rows can move as 16-byte-aligned bulk copies
   int flags;
+  // steady path, DPLUR (null otherwise): dq after compute_DQ_0 and the second iterate (dq
+  // layout), and the point-implicit chemistry's factors (interior planes): EPI LU and
+  // pivots, DA divisors
+  double *dq0, *dqk, *lu, *da;
+  unsigned char *piv;
 };
 
 constexpr int kZoneBulk = 1;

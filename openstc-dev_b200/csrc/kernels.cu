@@ -21,6 +21,7 @@ static __constant__ DevParam c_p;
 
 #include "chem.cuh"
 #include "mech_h2air9.cuh"
+#include "chem_implicit.cuh"
 #include "face.cuh"
 #include "kernels.cuh"
 #include "thermo.cuh"
@@ -1045,8 +1046,8 @@ static __global__ void store_last_kernel(DevZone z) {
 // the key (step << 44 | block << 34 | interior cell index; the step of the
 // call, at most 2^20 - 1, and a block below 1024) to an atomic minimum, so the
 // host learns the first failing cell of the earliest step.
-static __global__ void __launch_bounds__(256) residual_partial_kernel(DevZone z, double *partial, unsigned long long *bad,
-                                                               const int *step, int block) {
+__device__ __forceinline__ void residual_partial(const DevZone &z, double *partial, unsigned long long *bad, const int *step,
+                                                 int block) {
   const long long n = (long long)z.mx * z.my * z.mz;
   double s[4] = {0, 0, 0, 0};
   for (long long q = blockIdx.x * 256ll + threadIdx.x; q < n; q += 256ll * gridDim.x) {
@@ -1080,6 +1081,16 @@ static __global__ void __launch_bounds__(256) residual_partial_kernel(DevZone z,
   if (threadIdx.x == 0)
 #pragma unroll
     for (int l = 0; l < 4; ++l) partial[blockIdx.x * 4 + l] = red[l][0];
+}
+
+static __global__ void __launch_bounds__(256) residual_partial_kernel(DevZone z, double *partial, unsigned long long *bad,
+                                                               const int *step, int block) {
+  residual_partial(z, partial, bad, step, block);
+}
+
+// every zone of the table: zone blockIdx.y, its partials after those of the zones before it
+static __global__ void __launch_bounds__(256) residual_table_kernel(double *partial, unsigned long long *bad, const int *step) {
+  residual_partial(c_zones[blockIdx.y], partial + 4ll * gridDim.x * blockIdx.y, bad, step, blockIdx.y);
 }
 
 // sums n_part partials (fixed order) of every zone and writes sqrt(sum / n_total)
@@ -1369,7 +1380,10 @@ cudaError_t launch_steady(SteadyOp op, const DevZone &z, const SteadyArgs &a, co
   const dim3 blk(32, 8), blk4(32, 4);
   switch (op) {
     case SteadyOp::ChemImplicit:
-      chem_implicit_kernel<NS><<<plane_grid(z.mx, z.my, z.mz, blk4), blk4, 0, s>>>(z);
+      if (a.spec && NS == mech_h2air9::NS)
+        chem_implicit_kernel<NS, NS == mech_h2air9::NS><<<plane_grid(z.mx, z.my, z.mz, blk4), blk4, 0, s>>>(z);
+      else
+        chem_implicit_kernel<NS, 0><<<plane_grid(z.mx, z.my, z.mz, blk4), blk4, 0, s>>>(z);
       break;
     case SteadyOp::UpdateBv:
       update_bv_kernel<NS><<<plane_grid(z.mx, z.my, z.mz, blk), blk, 0, s>>>(z);
@@ -1378,13 +1392,19 @@ cudaError_t launch_steady(SteadyOp op, const DevZone &z, const SteadyArgs &a, co
       turb_implicit_kernel<<<plane_grid(z.mx, z.my, z.mz, blk), blk, 0, s>>>(z);
       break;
     case SteadyOp::DplurDq0:
-      dplur_dq0_kernel<NS><<<plane_grid(z.mx, z.my, z.mz, blk4), blk4, 0, s>>>(z, a);
+      if (a.spec && NS == mech_h2air9::NS)
+        dplur_dq0_kernel<NS, NS == mech_h2air9::NS><<<plane_grid(z.mx, z.my, z.mz, blk4), blk4, 0, s>>>(z, a);
+      else
+        dplur_dq0_kernel<NS, 0><<<plane_grid(z.mx, z.my, z.mz, blk4), blk4, 0, s>>>(z, a);
       break;
     case SteadyOp::DplurSweep:
-      dplur_sweep_kernel<NS><<<plane_grid(z.mx, z.my, z.mz, blk4), blk4, 0, s>>>(z, a);
+      if (a.spec && NS == mech_h2air9::NS)
+        dplur_sweep_kernel<NS, NS == mech_h2air9::NS><<<plane_grid(z.mx, z.my, z.mz, blk4), blk4, 0, s>>>(z, a);
+      else
+        dplur_sweep_kernel<NS, 0><<<plane_grid(z.mx, z.my, z.mz, blk4), blk4, 0, s>>>(z, a);
       break;
     case SteadyOp::DplurFinish:
-      dplur_finish_kernel<NS><<<plane_grid(z.mx, z.my, z.mz, blk), blk, 0, s>>>(z, a.dq_in);
+      dplur_finish_kernel<NS><<<plane_grid(z.mx, z.my, z.mz, blk), blk, 0, s>>>(z);
       break;
     case SteadyOp::WallDqZero: {
       if (!wall) return cudaErrorInvalidValue;
@@ -1392,12 +1412,44 @@ cudaError_t launch_steady(SteadyOp op, const DevZone &z, const SteadyArgs &a, co
       const int n0 = b.re[0] - b.rs[0] + 1, n1 = b.re[1] - b.rs[1] + 1, n2 = b.re[2] - b.rs[2] + 1;
       const dim3 wb(n0 >= 32 ? 32 : (n0 >= 8 ? 8 : 1), n1 >= 8 ? 8 : 1);
       wall_dq_zero_kernel<NS><<<dim3((n0 + wb.x - 1) / wb.x, (n1 + wb.y - 1) / wb.y, n2), wb, 0, s>>>(
-          z, b, a.dq_out);
+          z, b, a.buf);
       break;
     }
   }
   return cudaGetLastError();
 }
+
+template <int NS>
+cudaError_t launch_steady_table(SteadyOp op, const CellTable &tab, const SteadyArgs &a, cudaStream_t s) {
+  constexpr bool H = NS == mech_h2air9::NS;
+  const bool spec = a.spec && H;
+  switch (op) {
+    case SteadyOp::ChemImplicit:
+      return spec ? launch_table(tab, ChemImplicitOp<NS, H>{}, s) : launch_table(tab, ChemImplicitOp<NS, 0>{}, s);
+    case SteadyOp::UpdateBv: return launch_table(tab, UpdateBvOp<NS>{}, s);
+    case SteadyOp::TurbImplicit: return launch_table(tab, TurbImplicitOp<NS>{}, s);
+    case SteadyOp::DplurDq0:
+      return spec ? launch_table(tab, DplurDq0Op<NS, H>{a}, s) : launch_table(tab, DplurDq0Op<NS, 0>{a}, s);
+    case SteadyOp::DplurSweep:
+      return spec ? launch_table(tab, DplurSweepOp<NS, H>{a}, s) : launch_table(tab, DplurSweepOp<NS, 0>{a}, s);
+    case SteadyOp::DplurFinish: return launch_table(tab, DplurFinishOp<NS>{}, s);
+    default: return cudaErrorInvalidValue;
+  }
+}
+
+#ifndef OSTC_NS_UNIT
+// the zones of this unit's table (every context uploads it)
+cudaError_t launch_wall_zero_table(const CellTable &tab, const BcFace *faces, int buf, cudaStream_t s) {
+  if (tab.n <= 0) return cudaSuccess;
+  wall_dq_zero_table_kernel<<<tab.n < 4096 ? tab.n : 4096, dim3(32, 8), 0, s>>>(tab.tiles, tab.n, faces, buf);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_residual_table(int n_zones, const CellArgs &a, cudaStream_t s) {
+  residual_table_kernel<<<dim3(a.n_part, n_zones), 256, 0, s>>>(a.partial, a.bad, a.step);
+  return cudaGetLastError();
+}
+#endif  // OSTC_NS_UNIT
 
 template <int NS>
 cudaError_t launch_chem_integrator(int n, const double *T, const double *p, const double *Y, const double *dt,
@@ -1505,6 +1557,7 @@ cudaError_t upload_param(const DevParam &p, int ns, int nt, cudaStream_t s) {
   template cudaError_t launch_interface_waves<NS>(const Iface *, const WavePlan &, int, WaveSync *, cudaStream_t); \
   template cudaError_t launch_interface<NS>(const DevZone &, const DevZone &, const Iface &, int, cudaStream_t); \
   template cudaError_t launch_steady<NS>(SteadyOp, const DevZone &, const SteadyArgs &, const BcFace *, cudaStream_t); \
+  template cudaError_t launch_steady_table<NS>(SteadyOp, const CellTable &, const SteadyArgs &, cudaStream_t);          \
   template cudaError_t launch_chem_integrator<NS>(int, const double *, const double *, const double *, const double *, \
                                                   double *, double *, cudaStream_t);                                  \
   template cudaError_t launch_chem_surrogate<NS>(const mlp::Net &, int, const double *, const double *, const double *, \

@@ -93,13 +93,11 @@ struct CellArgs {
 // the steady path (steady.cuh)
 enum class SteadyOp { ChemImplicit, UpdateBv, DplurDq0, DplurSweep, DplurFinish, WallDqZero, TurbImplicit };
 struct SteadyArgs {
-  const double *dq_in = nullptr;  // DPLUR sweep: current iterate (dq layout)
-  double *dq_out = nullptr;       // DPLUR sweep: next iterate
-  double *dq0 = nullptr;          // DPLUR: dq after compute_DQ_0 (dq layout)
-  double *lu = nullptr;           // DPLUR + EPI: NS*NS interior planes of LU factors
-  unsigned char *piv = nullptr;   // DPLUR + EPI: NS interior planes of pivot rows
-  double *da = nullptr;           // DPLUR + DA: NS interior planes of diag - dt J_ll
-  int final_div = 0;              // DPLUR sweep: write (dq0 + ...) / dt_local into dq_out
+  // DPLUR's iterate buffer of the op (0: dq, 1: dqk): the one DplurDq0 writes, DplurSweep
+  // reads (it writes the other) and WallDqZero clears
+  int buf = 0;
+  int spec = 0;       // the mechanism's own chemistry (chem_implicit.cuh)
+  int final_div = 0;  // DPLUR sweep: write (dq0 + ...) / dt_local
 };
 
 // part 0: the face flux of the flow; 1: its inviscid half alone; 2: its
@@ -168,6 +166,13 @@ template <int NS>
 cudaError_t launch_interface(const DevZone &self, const DevZone &tar, const Iface &f, int with_cv, cudaStream_t s);
 template <int NS>
 cudaError_t launch_steady(SteadyOp op, const DevZone &z, const SteadyArgs &a, const BcFace *wall, cudaStream_t s);
+// the same over a tile table of (32 x 8)-thread interior tiles, and the wall clearing
+// over {face, a, b, 0} tiles of the wall faces in the device records
+template <int NS>
+cudaError_t launch_steady_table(SteadyOp op, const CellTable &tab, const SteadyArgs &a, cudaStream_t s);
+cudaError_t launch_wall_zero_table(const CellTable &tab, const BcFace *faces, int buf, cudaStream_t s);
+// residual partials of every zone of the uploaded table: n_part CTAs a zone
+cudaError_t launch_residual_table(int n_zones, const CellArgs &a, cudaStream_t s);
 template <int NS>
 cudaError_t launch_chem_integrator(int n, const double *T, const double *p, const double *Y, const double *dt,
                                    double *dY, double *dT, cudaStream_t s);

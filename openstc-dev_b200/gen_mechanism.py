@@ -68,7 +68,8 @@ def generate(mech) -> str:
     w("    cre[l] = 0;")
     w("    des[l] = 0;")
     w("  }")
-    for r in range(nr):
+    def rates(r):
+        """q1, q2 of reaction r (the body of a scope)"""
         ty = int(rt[r])
         eq = " + ".join(("%d %s" % (nuf[r, l], mech.names[l])).replace("1 ", "") for l in range(ns) if nuf[r, l])
         eqb = " + ".join(("%d %s" % (nub[r, l], mech.names[l])).replace("1 ", "") for l in range(ns) if nub[r, l])
@@ -130,6 +131,9 @@ def generate(mech) -> str:
                 w("    q2 *= %s;" % f)
         w("    q1 *= kf;")
         w("    q2 %s;" % ("*= kb" if ty != 0 else "= 0.0"))
+
+    for r in range(nr):
+        rates(r)
         def term(q, k):
             return q if k == 1 else "%s * %s" % (q, _lit(k))
 
@@ -147,6 +151,50 @@ def generate(mech) -> str:
         w("  }")
     w("#pragma unroll")
     w("  for (int l = 0; l < NS; ++l) om[l] = cre[l] * (c_p.mw[l] * 1e+3) - des[l] * (c_p.mw[l] * 1e+3);")
+    w("}")
+    w("")
+    # the chemical Jacobian over the species that take part in a reaction
+    act = [l for l in range(ns) if nuf[:, l].any() or nub[:, l].any()]
+    w("// species that take part in a reaction")
+    w("constexpr int NA = %d;" % len(act))
+    w("__host__ __device__ constexpr int active(int m) {")
+    w("  constexpr int a[NA] = {%s};" % ", ".join(map(str, act)))
+    w("  return a[m];")
+    w("}")
+    w("")
+    w("// net molar production wd[NA] (mol/(cm^3 s)) and its sensitivities")
+    w("// Z[m][n] = sum_r (nu''_m - nu'_m) (nu'_n q1 - nu''_n q2) over the active species:")
+    w("// d omega_m / d(rho Y_n) = 1e3 W_m Z[m][n] / (rho Y_n) (chem.cuh: chemistry_jacobian).")
+    w("// Each reaction adds to the entries of its own species only, and every index is a")
+    w("// literal, so Z stays in registers.")
+    w("__device__ __forceinline__ void production_jacobian(double rho, double t, const double *Y, double *wd,")
+    w("                                                    double (&Z)[NA][NA]) {")
+    w("  double c[NS], g[NS];")
+    w("  double lnT, invT, ln_temp_t;")
+    w("  chemistry_setup<NS>(rho, t, Y, c, g, lnT, invT, ln_temp_t);")
+    w("#pragma unroll")
+    w("  for (int m = 0; m < NA; ++m) {")
+    w("    wd[m] = 0;")
+    w("#pragma unroll")
+    w("    for (int n = 0; n < NA; ++n) Z[m][n] = 0;")
+    w("  }")
+
+    def add(to, k, q):
+        if k:
+            w("    %s %s= %s;" % (to, "+" if k > 0 else "-", q if abs(k) == 1 else "%s * %s" % (_lit(abs(k)), q)))
+
+    for r in range(nr):
+        rates(r)
+        w("    const double net = q1 - q2;")
+        for l in act:
+            add("wd[%d]" % act.index(l), int(nub[r, l] - nuf[r, l]), "net")
+        for n in act:
+            for m in act:
+                k = int(nub[r, m] - nuf[r, m])
+                add("Z[%d][%d]" % (act.index(m), act.index(n)), k * int(nuf[r, n]), "q1")
+                if rt[r] != 0:
+                    add("Z[%d][%d]" % (act.index(m), act.index(n)), -k * int(nub[r, n]), "q2")
+        w("  }")
     w("}")
     w("")
     w("}  // namespace mech_h2air9")
