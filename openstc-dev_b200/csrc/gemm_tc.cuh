@@ -36,7 +36,9 @@ struct TcGemmArgs {
   int M, N, K;             // N % 16 == 0, 16 <= N <= 256, K % 16 == 0
   int k_per_split;         // K of one blockIdx.y (a multiple of TC_BK)
   const float *bias;       // per column, or null (stored results only)
-  __nv_bfloat16 *act;      // bf16 silu(C) [M][ldc], or null
+  __nv_bfloat16 *act;      // bf16 silu(C) [M][ldc] (16-byte rows, N % 32 == 0), or null
+  __nv_bfloat16 *act_t;    // with act: its transpose [N][ldt], zero in columns M .. ldt - 1
+  int ldt;                 // a multiple of 16
   int atomic;              // add into C (C pre-zeroed) instead of storing
   int *err;                // set when a bounded wait ran out
 };
@@ -170,6 +172,32 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(TcGemmArgs g) {
 #pragma unroll
       for (int j = 0; j < 32; ++j)
         if (j < w) tile[lane * 33 + j] = v[j];
+      // the activations, from registers (lane = row; w = 32 here): a row's 32 columns as
+      // four 16-byte stores, and transposed (the K-major operand of the weight gradient),
+      // where a column's 32 rows are 64 contiguous bytes: neighbouring lanes exchange rows
+      // so that each stores two (even lanes of column j, odd lanes of column j + 1), zeros
+      // up to the padded length
+      if (g.act) {
+        const bool row = r0 + lane < g.M;
+        unsigned own[16];  // columns j, j + 1 of this row
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) {
+          const float y0 = v[j] + (g.bias ? g.bias[c0 + j] : 0.f), y1 = v[j + 1] + (g.bias ? g.bias[c0 + j + 1] : 0.f);
+          own[j / 2] = row ? pack_bf16(silu_tc(y0), silu_tc(y1)) : 0u;
+        }
+        if (row) {
+          uint4 *o = reinterpret_cast<uint4 *>(g.act + (long long)(r0 + lane) * g.ldc + c0);
+#pragma unroll
+          for (int q = 0; q < 4; ++q) o[q] = make_uint4(own[4 * q], own[4 * q + 1], own[4 * q + 2], own[4 * q + 3]);
+        }
+        __nv_bfloat16 *ot = g.act_t + (long long)(c0 + (lane & 1)) * g.ldt + r0 + (lane & ~1);
+#pragma unroll
+        for (int j = 0; j < 32; j += 2) {
+          const unsigned oth = __shfl_xor_sync(0xffffffffu, own[j / 2], 1);
+          const unsigned x = lane & 1 ? __byte_perm(oth, own[j / 2], 0x7632) : __byte_perm(own[j / 2], oth, 0x5410);
+          if (r0 + lane < g.ldt) *reinterpret_cast<unsigned *>(ot + (long long)j * g.ldt) = x;
+        }
+      }
       __syncwarp();
       if (lane < w) {
         const float bias = (!g.atomic && g.bias) ? g.bias[c0 + lane] : 0.f;
@@ -179,9 +207,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(TcGemmArgs g) {
           if (g.atomic) {
             atomicAdd(g.c + o, x);
           } else {
-            const float y = x + bias;
-            g.c[o] = y;
-            if (g.act) g.act[o] = __float2bfloat16_rn(silu_tc(y));
+            g.c[o] = x + bias;
           }
         }
       }
@@ -198,6 +224,8 @@ inline cudaError_t gemm_tc(const TcGemmArgs &a0, int splits, cudaStream_t s) {
   TcGemmArgs a = a0;
   if (a.N % 16 || a.N < 16 || a.N > 256 || a.K % 16 || a.K <= 0 || a.M <= 0 || a.lda % 8 || a.ldb % 8 ||
       (reinterpret_cast<uintptr_t>(a.a) & 15) || (reinterpret_cast<uintptr_t>(a.b) & 15) || !a.err)
+    return cudaErrorInvalidValue;
+  if (a.act && (!a.act_t || a.N % 32 || a.ldc % 8 || a.ldt % 16 || (reinterpret_cast<uintptr_t>(a.act) & 15)))
     return cudaErrorInvalidValue;
   splits = splits < 1 ? 1 : splits;
   a.k_per_split = ((a.K + splits - 1) / splits + TC_BK - 1) / TC_BK * TC_BK;

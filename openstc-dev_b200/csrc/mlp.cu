@@ -16,7 +16,8 @@
 //                        gradients dZ^T X (against the transposed gradients
 //                        and activations, split over the batch with FP32
 //                        atomics);
-//   transpose / loss / SiLU-backward / column-sum / Adam kernels for the rest.
+//   SiLU backward with the transposed gradients and bias sums; transpose, loss,
+//   column-sum and Adam kernels for the rest.
 // gemm_bf16_kernel (mma.sync m16n8k16, generic strides) serves the
 // reference forward of ostc_surrogate_forward.
 // The fused inference kernel of the hot path (tcgen05, TMEM accumulators)
@@ -211,16 +212,59 @@ __global__ void loss_grad_kernel(const float *z4, const float *y, int n, float *
   if (threadIdx.x == 0) atomicAdd(loss_sum, red[0]);
 }
 
-// dZ = dA * silu'(Z), FP32 and BF16 copies
-__global__ void silu_backward_kernel(const float *da, const float *z, long long count, float *dz,
-                                     __nv_bfloat16 *dzb) {
-  const long long e = blockIdx.x * 256ll + threadIdx.x;
-  if (e >= count) return;
-  const float zz = z[e];
-  const float sg = 1.0f / (1.0f + __expf(-zz));
-  const float d = da[e] * sg * (1.0f + zz * (1.0f - sg));
-  dz[e] = d;
-  dzb[e] = __float2bfloat16_rn(d);
+// dZ = dA * silu'(Z) of a hidden layer: the BF16 copy, its transpose dzt [256][ldt] (the
+// K-major operand of the weight gradient, zero from row n to ldt) and the bias gradient's
+// column sums (added into db, from the FP32 values). Bound by HBM: dA and Z in, two BF16
+// copies out. One CTA takes 64 columns of `rows` rows, 64 x 64 at a time: 16-byte loads,
+// 8-byte stores of the rows, the transposed tile through shared memory in 16-byte stores.
+// The FP32 dZ is not written: with separate SiLU, transpose and column-sum kernels a layer
+// took 115 us at 65536 rows, now 45.
+__global__ void __launch_bounds__(256) silu_backward_kernel(const float *da, const float *z, int n, __nv_bfloat16 *dzb,
+                                                            __nv_bfloat16 *dzt, int ldt, float *db, int rows) {
+  __shared__ __align__(16) __nv_bfloat16 t[64][72];  // rows of 144 bytes: 16-byte aligned, banks apart
+  __shared__ float red[16][64];
+  const int cx = threadIdx.x & 15, ry = threadIdx.x >> 4;  // 4 columns, rows ry + 16 i
+  const int c0 = blockIdx.y * 64;
+  const int out_c = threadIdx.x >> 2, out_r = (threadIdx.x & 3) * 16;
+  float sum[4] = {0.f, 0.f, 0.f, 0.f};
+  const int end = min(ldt, (int)(blockIdx.x + 1) * rows);
+  for (int r0 = blockIdx.x * rows; r0 < end; r0 += 64) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int r = r0 + ry + 16 * i;
+      float d[4] = {0.f, 0.f, 0.f, 0.f};
+      if (r < n) {
+        const long long o = (long long)r * NH + c0 + 4 * cx;
+        const float4 a = *(const float4 *)(da + o), v = *(const float4 *)(z + o);
+        const float aa[4] = {a.x, a.y, a.z, a.w}, zz[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float sg = 1.0f / (1.0f + __expf(-zz[e]));
+          d[e] = aa[e] * sg * (1.0f + zz[e] * (1.0f - sg));
+          sum[e] += d[e];
+        }
+        *(uint2 *)(dzb + o) = make_uint2(tc::pack_bf16(d[0], d[1]), tc::pack_bf16(d[2], d[3]));
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) t[4 * cx + e][ry + 16 * i] = __float2bfloat16_rn(d[e]);
+    }
+    __syncthreads();
+    if (r0 + out_r < ldt) {  // ldt is a multiple of 16
+      uint4 *o = (uint4 *)(dzt + (long long)(c0 + out_c) * ldt + r0 + out_r);
+      o[0] = *(const uint4 *)&t[out_c][out_r];
+      o[1] = *(const uint4 *)&t[out_c][out_r + 8];
+    }
+    __syncthreads();
+  }
+#pragma unroll
+  for (int e = 0; e < 4; ++e) red[ry][4 * cx + e] = sum[e];
+  __syncthreads();
+  if (threadIdx.x < 64) {
+    float s = 0.f;
+#pragma unroll
+    for (int q = 0; q < 16; ++q) s += red[q][threadIdx.x];
+    atomicAdd(db + c0 + threadIdx.x, s);
+  }
 }
 
 // out[c][b] = in[b][c] for b < rows, 0 for rows <= b < ldo (a K-major operand
@@ -335,11 +379,12 @@ struct ostc_surrogate {
   unsigned char *mask = nullptr;  // 1 where the padded slot is a real parameter
   // activations of a training batch
   __nv_bfloat16 *x0 = nullptr, *a[3] = {nullptr, nullptr, nullptr}, *dzb[4] = {nullptr, nullptr, nullptr, nullptr};
-  float *z[4] = {nullptr, nullptr, nullptr, nullptr}, *dz[4] = {nullptr, nullptr, nullptr, nullptr};
+  float *z[4] = {nullptr, nullptr, nullptr, nullptr}, *dz3 = nullptr;
   float *da = nullptr, *loss = nullptr;
-  // K-major operands of the backward GEMMs: transposed gradients and
-  // activations ([256][batch padded to 16]) and transposed weights of layers 2..4
-  __nv_bfloat16 *tg = nullptr, *ta = nullptr, *wt = nullptr;
+  // K-major operands of the backward GEMMs: transposed gradients, inputs and
+  // activations ([256][batch padded to 16]; the forward writes the activations') and
+  // transposed weights of layers 2..4
+  __nv_bfloat16 *tg = nullptr, *ta[4] = {nullptr, nullptr, nullptr, nullptr}, *wt = nullptr;
   int *err = nullptr;  // set by a tensor-core kernel whose bounded wait ran out
   Checks *checks = nullptr;  // device copy of the acceptance tests
   int *list = nullptr, *count = nullptr;
@@ -401,6 +446,7 @@ ostc_status forward(ostc_surrogate *s, int n, cudaStream_t st) {
     const int k = l == 0 ? KIN : NH, nn = l == 3 ? NOUTP : NH;
     g.a = in[l], g.lda = k, g.b = wl[l], g.ldb = k;
     g.c = s->z[l], g.ldc = nn, g.M = n, g.N = nn, g.K = k, g.bias = bl[l], g.act = l < 3 ? s->a[l] : nullptr;
+    g.act_t = l < 3 ? s->ta[l + 1] : nullptr, g.ldt = (n + 15) / 16 * 16;
     g.err = s->err;
     SK(gemm_tc(g, 1, st));
   }
@@ -434,33 +480,30 @@ ostc_status backward(ostc_surrogate *s, const float *y, int n, cudaStream_t st) 
   const Net &w = s->net;
   SK(cudaMemsetAsync(s->loss, 0, sizeof(float), st));
   SK(cudaMemsetAsync(s->grad, 0, sizeof(float) * NPAR, st));
-  loss_grad_kernel<<<blocks((long long)n * NOUTP), 256, 0, st>>>(s->z[3], y, n, s->dz[3], s->dzb[3], s->loss);
+  loss_grad_kernel<<<blocks((long long)n * NOUTP), 256, 0, st>>>(s->z[3], y, n, s->dz3, s->dzb[3], s->loss);
   SK(cudaGetLastError());
   const int np = (n + 15) / 16 * 16;  // the batch as a K, padded with zero columns
-  const __nv_bfloat16 *acts[4] = {s->x0, s->a[0], s->a[1], s->a[2]};
   const int kin[4] = {KIN, NH, NH, NH}, nout[4] = {NH, NH, NH, NOUTP};
   const long long offw[4] = {OFF_W1, OFF_W2, OFF_W3, OFF_W4}, offb[4] = {OFF_B1, OFF_B2, OFF_B3, OFF_B4};
   const __nv_bfloat16 *wl[4] = {w.w1(), w.w2(), w.w3(), w.w4()};
   const dim3 tb(32, 8);
+  transpose_bf16_kernel<<<dim3((np + 31) / 32, (KIN + 31) / 32), tb, 0, st>>>(s->x0, n, KIN, KIN, s->ta[0], np);
+  SK(cudaGetLastError());
+  transpose_bf16_kernel<<<dim3((np + 31) / 32, (NOUTP + 31) / 32), tb, 0, st>>>(s->dzb[3], n, NOUTP, NOUTP, s->tg, np);
+  SK(cudaGetLastError());
+  colsum_kernel<<<dim3((NOUTP + 31) / 32, std::max(1, std::min(n / 64, 256))), 256, 0, st>>>(s->dz3, n, NOUTP,
+                                                                                            s->grad + OFF_B4);
+  SK(cudaGetLastError());
   for (int l = 3; l >= 0; --l) {
     // weight gradient dW[n_out][k_in] = sum_b dZ[b][n_out] A[b][k_in]: dZ^T and A^T
     // as K-major operands, split over the batch so that about two CTAs per SM run
-    transpose_bf16_kernel<<<dim3((np + 31) / 32, (nout[l] + 31) / 32), tb, 0, st>>>(s->dzb[l], n, nout[l], nout[l],
-                                                                                   s->tg, np);
-    SK(cudaGetLastError());
-    transpose_bf16_kernel<<<dim3((np + 31) / 32, (kin[l] + 31) / 32), tb, 0, st>>>(acts[l], n, kin[l], kin[l], s->ta,
-                                                                                  np);
-    SK(cudaGetLastError());
     TcGemmArgs g{};
-    g.a = s->tg, g.lda = np, g.b = s->ta, g.ldb = np;
+    g.a = s->tg, g.lda = np, g.b = s->ta[l], g.ldb = np;
     g.c = s->grad + offw[l], g.ldc = kin[l], g.M = nout[l], g.N = kin[l], g.K = np, g.atomic = 1;
     g.err = s->err;
     const int mt = (nout[l] + 127) / 128;
     const int splits = std::max(1, std::min(np / 1024, 296 / mt));
     SK(gemm_tc(g, splits, st));
-    colsum_kernel<<<dim3((nout[l] + 31) / 32, std::max(1, std::min(n / 64, 256))), 256, 0, st>>>(
-        s->dz[l], n, nout[l], s->grad + offb[l]);
-    SK(cudaGetLastError());
     if (l == 0) break;
     // input gradient dA[b][k] = sum_n dZ[b][n] W[n][k], against W^T [k_in][n_out]
     __nv_bfloat16 *wt = s->wt + (long long)(l - 1) * NH * NH;
@@ -472,8 +515,10 @@ ostc_status backward(ostc_surrogate *s, const float *y, int n, cudaStream_t st) 
     h.c = s->da, h.ldc = NH, h.M = n, h.N = kin[l], h.K = nout[l];
     h.err = s->err;
     SK(gemm_tc(h, 1, st));
-    silu_backward_kernel<<<blocks((long long)n * NH), 256, 0, st>>>(s->da, s->z[l - 1], (long long)n * NH,
-                                                                     s->dz[l - 1], s->dzb[l - 1]);
+    // 256 rows a CTA (fewer sums to add up), or less so that about eight CTAs per SM run
+    const int rows = std::min(256, (np * (NH / 64) / 1184 + 63) / 64 * 64 + (np * (NH / 64) < 1184 ? 64 : 0));
+    silu_backward_kernel<<<dim3((np + rows - 1) / rows, NH / 64), 256, 0, st>>>(
+        s->da, s->z[l - 1], n, s->dzb[l - 1], s->tg, np, s->grad + offb[l - 1], rows);
     SK(cudaGetLastError());
   }
   return OSTC_OK;
@@ -505,7 +550,8 @@ ostc_status ostc_surrogate_create(int max_batch, unsigned long long seed, ostc_s
             dalloc(s, (void **)&s->x0, sizeof(__nv_bfloat16) * B * KIN) == cudaSuccess &&
             dalloc(s, (void **)&s->da, sizeof(float) * B * NH) == cudaSuccess &&
             dalloc(s, (void **)&s->tg, sizeof(__nv_bfloat16) * NH * ((B + 15) / 16 * 16)) == cudaSuccess &&
-            dalloc(s, (void **)&s->ta, sizeof(__nv_bfloat16) * NH * ((B + 15) / 16 * 16)) == cudaSuccess &&
+            dalloc(s, (void **)&s->ta[0], sizeof(__nv_bfloat16) * KIN * ((B + 15) / 16 * 16)) == cudaSuccess &&
+            dalloc(s, (void **)&s->dz3, sizeof(float) * B * NOUTP) == cudaSuccess &&
             dalloc(s, (void **)&s->wt, sizeof(__nv_bfloat16) * 3 * NH * NH) == cudaSuccess &&
             dalloc(s, (void **)&s->loss, sizeof(float)) == cudaSuccess &&
             dalloc(s, (void **)&s->err, sizeof(int)) == cudaSuccess &&
@@ -514,9 +560,10 @@ ostc_status ostc_surrogate_create(int max_batch, unsigned long long seed, ostc_s
   for (int l = 0; l < 4 && ok; ++l) {
     const long long w = l == 3 ? NOUTP : NH;
     ok = dalloc(s, (void **)&s->z[l], sizeof(float) * B * w) == cudaSuccess &&
-         dalloc(s, (void **)&s->dz[l], sizeof(float) * B * w) == cudaSuccess &&
          dalloc(s, (void **)&s->dzb[l], sizeof(__nv_bfloat16) * B * w) == cudaSuccess;
-    if (ok && l < 3) ok = dalloc(s, (void **)&s->a[l], sizeof(__nv_bfloat16) * B * NH) == cudaSuccess;
+    if (ok && l < 3)
+      ok = dalloc(s, (void **)&s->a[l], sizeof(__nv_bfloat16) * B * NH) == cudaSuccess &&
+           dalloc(s, (void **)&s->ta[l + 1], sizeof(__nv_bfloat16) * NH * ((B + 15) / 16 * 16)) == cudaSuccess;
   }
   if (!ok) {
     ostc_surrogate_destroy(s);
