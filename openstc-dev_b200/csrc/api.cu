@@ -1612,8 +1612,7 @@ ostc_status ostc_chem_surrogate(ostc_ctx *ctx, ostc_surrogate *sur, int n, const
   CK(launch_chem_surrogate<mlp::NIN - 3>(*surrogate_net(sur), n, T, p, Y, dt, dY, dT, w, S(stream)));
   if (n_fallback) {
     int h[2] = {0, 0};
-    CK(cudaMemcpyAsync(&h[0], w.count, sizeof(int), cudaMemcpyDeviceToHost, S(stream)));
-    CK(cudaMemcpyAsync(&h[1], w.err, sizeof(int), cudaMemcpyDeviceToHost, S(stream)));
+    CK(cudaMemcpyAsync(h, w.count, sizeof(h), cudaMemcpyDeviceToHost, S(stream)));  // count, err (mlp.cuh)
     CK(cudaStreamSynchronize(S(stream)));
     *n_fallback = h[0];
     if (h[1]) return fail(ctx, OSTC_ERR_TIMEOUT);

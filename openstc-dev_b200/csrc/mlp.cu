@@ -554,8 +554,7 @@ ostc_status ostc_surrogate_create(int max_batch, unsigned long long seed, ostc_s
             dalloc(s, (void **)&s->dz3, sizeof(float) * B * NOUTP) == cudaSuccess &&
             dalloc(s, (void **)&s->wt, sizeof(__nv_bfloat16) * 3 * NH * NH) == cudaSuccess &&
             dalloc(s, (void **)&s->loss, sizeof(float)) == cudaSuccess &&
-            dalloc(s, (void **)&s->err, sizeof(int)) == cudaSuccess &&
-            dalloc(s, (void **)&s->count, sizeof(int)) == cudaSuccess &&
+            dalloc(s, (void **)&s->count, 2 * sizeof(int)) == cudaSuccess &&
             dalloc(s, (void **)&s->checks, sizeof(Checks)) == cudaSuccess;
   for (int l = 0; l < 4 && ok; ++l) {
     const long long w = l == 3 ? NOUTP : NH;
@@ -569,6 +568,7 @@ ostc_status ostc_surrogate_create(int max_batch, unsigned long long seed, ostc_s
     ostc_surrogate_destroy(s);
     return OSTC_ERR_CUDA;
   }
+  s->err = s->count + 1;  // beside the fallback count, so that one copy reads both
   s->net.wf = s->master;
   s->net.checks = s->checks;
   // He-uniform initialisation from a seeded 64-bit LCG (biases zero)

@@ -69,7 +69,8 @@ struct Net {
 // the device parameters of a surrogate (mlp.cu), for the inference path
 const mlp::Net *surrogate_net(const ostc_surrogate *s);
 // per-call scratch of the surrogate chemistry step, for at least n states
-// (grown on demand): the fallback list and its counter, the error word, the
+// (grown on demand): the fallback list and its counter, the error word (the int
+// after the counter), the
 // standardised BF16 feature rows [n][16], the network's outputs [n][10] and
 // the training-envelope flags [n]
 struct ChemScratch {

@@ -159,7 +159,7 @@ static __global__ void __launch_bounds__(tc::THREADS, 1) surrogate_chem_kernel(m
 // the element-mass and internal-energy checks in FP32; a state outside the
 // envelope or failing a check goes to the fallback list (warp-aggregated)
 template <int NS>
-__global__ void __launch_bounds__(256, 2) chem_checks_kernel(int n, const double *T, const double *Y, const double *dt,
+__global__ void __launch_bounds__(256, 3) chem_checks_kernel(int n, const double *T, const double *Y, const double *dt,
                                                           const float *y, const unsigned char *env,
                                                           const double *scale, const mlp::Checks *ck, double *dY,
                                                           double *dT, int *list, int *count) {
