@@ -54,10 +54,29 @@ def test_forward_and_gradients_match_oracle(n):
     s.close()
 
 
-@pytest.mark.parametrize("n", [1, 127, 128, 5000, 300000])
+@pytest.mark.parametrize("n", [1, 17, 20005, 65536])
+def test_gradients_match_oracle_over_batches(n):
+    """Batches from one row to the training loop's: from about 19 000 rows on, a CTA of the
+    SiLU backward walks several 64-row tiles (its transposed tile reused, its column sums
+    carried on); 17 and 20 005 rows are padded."""
+    import torch
+
+    s = ostc.Surrogate(max_batch=n, seed=3)
+    p = s.params().astype(np.float64)
+    x, y = _data(n, 5)
+    g, loss = s.gradients(torch.from_numpy(x).cuda(), torch.from_numpy(y).cuda())
+    gref, lref = M.gradients(p, x.astype(np.float64), y.astype(np.float64))
+    assert abs(loss - lref) <= 1e-3 * lref
+    err = _per_tensor_err(g.astype(np.float64), gref)
+    assert max(err.values()) <= 2e-3, err
+    s.close()
+
+
+@pytest.mark.parametrize("n", [1, 63, 64, 65, 127, 128, 129, 5000, 300000])
 def test_tensor_core_forward_matches(n):
-    """The tcgen05 inference kernel (TMEM accumulators, 128-row tiles, ragged
-    last tile) against the mma.sync forward and the BF16-emulating oracle."""
+    """The tcgen05 inference kernel (TMEM accumulators, two groups a CTA with tiles of
+    64 states, ragged last tile, a group without one) against the mma.sync forward and
+    the BF16-emulating oracle."""
     import torch
 
     s = ostc.Surrogate(max_batch=max(n, 8), seed=11)
