@@ -492,8 +492,8 @@ __device__ __forceinline__ void inviscid_face_roe(const DevZone &z, int g0, doub
 // away from it (AWENO.cu: the other side takes them reversed). The weights
 // d_i (1 + tau / (eps + b_i)^2) are taken times the product of the three
 // (eps + b_i)^2, which cancels in the quotient: one division where the weights
-// one by one take four. The product stays in range for characteristic values
-// below 1e25.
+// one by one take four. The product grows with the twelfth power of the values
+// and stays in range below 1e22; the face scales larger ones (aweno_shift).
 __device__ __forceinline__ double weno5(double w0, double w1, double w2, double w3, double w4) {
   constexpr double t13 = 13.0 / 12, eps = 1e-6, d0 = 1.0 / 16, d1 = 5.0 / 8, d2 = 5.0 / 16;
   const double s0 = w0 + w2 - 2 * w1, s1 = w1 + w3 - 2 * w2, s2 = w2 + w4 - 2 * w3;
@@ -512,6 +512,22 @@ __device__ __forceinline__ void weno5_pair(const double v[6], double &vminus, do
   vplus = weno5(v[5], v[4], v[3], v[2], v[1]);
 }
 
+// 2^n
+__device__ __forceinline__ double exp2i(int n) { return __hiloint2double((1023 + n) << 20, 0); }
+
+// The shift n of a face whose characteristic values are reconstructed times 2^-n:
+// 0 unless a density of the stencil exceeds 2^50 (the values are densities times a
+// polynomial of the Mach number), so that ordinary faces only compare; else the
+// largest comes to 2^50, where eps is below the rounding of the squares as it was
+// before the shift. With the quotients one by one values up to 1e76 are in range;
+// in SI units none come near.
+__device__ __forceinline__ int aweno_shift(const double (&U)[6][5]) {
+  int top = __double2hiint(U[0][0]);
+#pragma unroll
+  for (int s = 1; s < 6; ++s) top = max(top, __double2hiint(U[s][0]));
+  return max((top >> 20) - (1023 + 50), 0);
+}
+
 // NT = 2 (SST): k and omega are not part of the reference's AWENO (quirk A3:
 // its WENO5 reads a 5-variable row stride); here their conservative values
 // rho k, rho omega are reconstructed component by component with the same
@@ -527,6 +543,7 @@ __device__ __forceinline__ void inviscid_face_aweno(const DevZone &z, int g0, do
 #pragma unroll
     for (int l = 0; l < 5; ++l) U[s][l] = cvl(z, g0 + (s - 2) * sd, l);
   const double pL = bvl(z, g0, 4), pR = bvl(z, g0 + sd, 4);
+  const int shift = aweno_shift(U);
   const double *cl = U[2], *cr = U[3];
   const double sl0 = sqrt(cl[0]), sr0 = sqrt(cr[0]), isum = 1.0 / (sl0 + sr0);
   // Roe weights over the densities
@@ -538,7 +555,8 @@ __device__ __forceinline__ void inviscid_face_aweno(const DevZone &z, int g0, do
   const double hm = wl * (cl[4] + pL) + wr * (cr[4] + pR);
   const double cm2 = gm1 * (hm - ekm);
   const double cm = sqrt(cm2);
-  const double ic2 = 1.0 / cm2, ic = cm * ic2, hc2 = 0.5 * ic2;
+  // the left eigenvectors carry the shift
+  const double one = exp2i(-shift), ic2 = one / cm2, ic = cm * ic2, hc2 = 0.5 * ic2;
   const int g1 = g0 + sd;
   double kx = 0.5 * (met(z, g0, 3 * DIR) + met(z, g1, 3 * DIR));
   double ky = 0.5 * (met(z, g0, 3 * DIR + 1) + met(z, g1, 3 * DIR + 1));
@@ -563,21 +581,21 @@ __device__ __forceinline__ void inviscid_face_aweno(const DevZone &z, int g0, do
           L[4] = gm1 * hc2;
           break;
         case 1:
-          L[0] = kx * (1 - alpha * ic2) - (kz * vm - ky * wm) * ic;
+          L[0] = kx * (one - alpha * ic2) - (kz * vm - ky * wm) * ic;
           L[1] = kx * gm1 * um * ic2;
           L[2] = (kx * gm1 * vm + kz * cm) * ic2;
           L[3] = (kx * gm1 * wm - ky * cm) * ic2;
           L[4] = -kx * gm1 * ic2;
           break;
         case 2:
-          L[0] = ky * (1 - alpha * ic2) - (kx * wm - kz * um) * ic;
+          L[0] = ky * (one - alpha * ic2) - (kx * wm - kz * um) * ic;
           L[1] = (ky * gm1 * um - kz * cm) * ic2;
           L[2] = ky * gm1 * vm * ic2;
           L[3] = (ky * gm1 * wm + kx * cm) * ic2;
           L[4] = -ky * gm1 * ic2;
           break;
         case 3:
-          L[0] = kz * (1 - alpha * ic2) - (ky * um - kx * vm) * ic;
+          L[0] = kz * (one - alpha * ic2) - (ky * um - kx * vm) * ic;
           L[1] = (kz * gm1 * um + ky * cm) * ic2;
           L[2] = (kz * gm1 * vm - kx * cm) * ic2;
           L[3] = kz * gm1 * wm * ic2;
@@ -619,6 +637,10 @@ __device__ __forceinline__ void inviscid_face_aweno(const DevZone &z, int g0, do
       }
     }
   }
+  if (shift) {
+#pragma unroll
+    for (int m = 0; m < 5; ++m) ql[m] *= exp2i(shift), qr[m] *= exp2i(shift);
+  }
   double pl[NV + 4], pr[NV + 4];
   const double il = 1.0 / ql[0];
   pl[0] = ql[0];
@@ -645,8 +667,12 @@ __device__ __forceinline__ void inviscid_face_aweno(const DevZone &z, int g0, do
     double v[6];
 #pragma unroll
     for (int s = 0; s < 6; ++s) v[s] = cvl(z, g0 + (s - 2) * sd, 5 + t);
+    if (shift)
+#pragma unroll
+      for (int s = 0; s < 6; ++s) v[s] *= exp2i(-shift);
     double vmn = 0, vpl = 0;
     if (c_p.reconstruction == 4) weno5_pair(v, vmn, vpl);
+    if (shift) vmn *= exp2i(shift), vpl *= exp2i(shift);
     pl[5 + t] = vmn * il;
     pr[5 + t] = vpl * ir;
   }
