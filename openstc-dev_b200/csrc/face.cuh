@@ -110,6 +110,19 @@ __device__ __forceinline__ double minmod(double a, double b) {
   return (a < 0) != (b < 0) ? 0.0 : m;
 }
 
+// a / b where r = 1 / b to a few rounding errors is at hand: the product with
+// one correction by its residual, as accurate as a division (P. Markstein, IBM
+// J. Res. Dev. 34, 1990), three operations instead of about twenty. Used where
+// plain products with r showed in a residual's error against extended precision
+// (2-norms): the density's with AUSM+, 9.4e-15 with divisions or corrected,
+// 9.8e-15 without (nine species 6.2e-15 and 7.4e-15); AWENO's 2.37e-14 with
+// divisions, 2.45e-14 without, 2.38e-14 with the velocities corrected (and p / rho
+// from the specific energy).
+__device__ __forceinline__ double quotient(double a, double b, double r) {
+  const double q = a * r;
+  return fma(fma(-q, b, a), r, q);
+}
+
 // ---------------------------------------------------------------------------
 // Riemann solvers on reconstructed states (pl/pr: NV primitive values, then
 // total energy at NV, gamma at NV+1, total enthalpy (E + p) / rho at NV+2 and
@@ -124,9 +137,9 @@ __device__ __forceinline__ void ausm_plus(const double *pl, const double *pr, do
   const double gk = sqrt(k1 * k1 + k2 * k2 + k3 * k3);
   const double gl = MIXG ? pl[NV + 1] : gamma_air, gr = MIXG ? pr[NV + 1] : gamma_air;
   const double c = 0.5 * (sqrt(gl * pl[NV + 3]) + sqrt(gr * pr[NV + 3]));
-  const double igc = 1.0 / (gk * c);
-  const double mlm = (k1 * pl[1] + k2 * pl[2] + k3 * pl[3]) * igc;
-  const double mrm = (k1 * pr[1] + k2 * pr[2] + k3 * pr[3]) * igc;
+  const double igc = 1.0 / (gk * c), igk = igc * c, ic = igc * gk;
+  const double mlm = quotient(quotient(k1 * pl[1] + k2 * pl[2] + k3 * pl[3], gk, igk), c, ic);
+  const double mrm = quotient(quotient(k1 * pr[1] + k2 * pr[2] + k3 * pr[3], gk, igk), c, ic);
   double mlp, mrn, plp, prn;
   constexpr double alpha = 3 / 16.0;
   if (fabs(mlm) > 1) {
@@ -644,24 +657,24 @@ __device__ __forceinline__ void inviscid_face_aweno(const DevZone &z, int g0, do
   double pl[NV + 4], pr[NV + 4];
   const double il = 1.0 / ql[0];
   pl[0] = ql[0];
-  pl[1] = ql[1] * il;
-  pl[2] = ql[2] * il;
-  pl[3] = ql[3] * il;
-  pl[4] = gm1 * (ql[4] - 0.5 * (pl[1] * pl[1] + pl[2] * pl[2] + pl[3] * pl[3]) * ql[0]);
+  pl[1] = quotient(ql[1], ql[0], il);
+  pl[2] = quotient(ql[2], ql[0], il);
+  pl[3] = quotient(ql[3], ql[0], il);
+  pl[NV + 3] = gm1 * (ql[4] * il - 0.5 * (pl[1] * pl[1] + pl[2] * pl[2] + pl[3] * pl[3]));
+  pl[4] = pl[NV + 3] * ql[0];
   pl[NV] = ql[4];
   pl[NV + 1] = gamma_air;
-  pl[NV + 2] = (ql[4] + pl[4]) * il;
-  pl[NV + 3] = pl[4] * il;
+  pl[NV + 2] = ql[4] * il + pl[NV + 3];
   const double ir = 1.0 / qr[0];
   pr[0] = qr[0];
-  pr[1] = qr[1] * ir;
-  pr[2] = qr[2] * ir;
-  pr[3] = qr[3] * ir;
-  pr[4] = gm1 * (qr[4] - 0.5 * (pr[1] * pr[1] + pr[2] * pr[2] + pr[3] * pr[3]) * qr[0]);
+  pr[1] = quotient(qr[1], qr[0], ir);
+  pr[2] = quotient(qr[2], qr[0], ir);
+  pr[3] = quotient(qr[3], qr[0], ir);
+  pr[NV + 3] = gm1 * (qr[4] * ir - 0.5 * (pr[1] * pr[1] + pr[2] * pr[2] + pr[3] * pr[3]));
+  pr[4] = pr[NV + 3] * qr[0];
   pr[NV] = qr[4];
   pr[NV + 1] = gamma_air;
-  pr[NV + 2] = (qr[4] + pr[4]) * ir;
-  pr[NV + 3] = pr[4] * ir;
+  pr[NV + 2] = qr[4] * ir + pr[NV + 3];
 #pragma unroll
   for (int t = 0; t < NT; ++t) {  // componentwise WENO5 of rho k, rho omega
     double v[6];
