@@ -253,7 +253,7 @@ __device__ __forceinline__ void lax_friedrichs(const double *pl, const double *p
   const double gradK = sqrt(kx * kx + ky * ky + kz * kz);
   const double Ukl = pl[1] * kx + pl[2] * ky + pl[3] * kz;
   const double Ukr = pr[1] * kx + pr[2] * ky + pr[3] * kz;
-  const double cl = sqrt(gamma_air * pl[4] / pl[0]), cr = sqrt(gamma_air * pr[4] / pr[0]);
+  const double cl = sqrt(gamma_air * pl[NV + 3]), cr = sqrt(gamma_air * pr[NV + 3]);
   const double sr = fmax(fabs(Ukl) + cl * gradK, fabs(Ukr) + cr * gradK);
   const double hj = 0.5 * jac_ave;
   const double rUl = pl[0] * Ukl, rUr = pr[0] * Ukr;
