@@ -780,18 +780,25 @@ void build_devparam(const ostc_param *p, DevParam &d) {
 
 // default tile shapes of a context's sweeps (before the autotuner or
 // ostc_set_tile choose). The build by what it is bound by, with flux times in us
-// of the x, y, z sweeps against the 255-register plane kernels that ran before:
+// of the x, y, z sweeps against the 255-register plane kernels:
 //  - staged where two CTAs fit an SM's shared memory, for mixtures (97 x 113 x 61,
 //    9 species: 253 / 313 / 315 against 549 / 760 / 737; 4 species 207 / 231 / 236
-//    against 231 / 310 / 306) and SST (9 blocks of air: 145 / 174 / 177 against
-//    264 / 375 / 400); one staged CTA per SM loses (12 species, y and z: 322 against
-//    267 for the 128-register plane kernel);
+//    against 231 / 310 / 306); one staged CTA per SM loses (12 species, y and z: 322
+//    against 267 for the 128-register plane kernel);
+//    Air with SST likewise (96 x 96 x 96: 156 / 145 / 141 against 334 / 352 / 377), but
+//    where its blocks have both odd and even rows, which the staged kernels take in a
+//    launch each: then plane kernels of 80 registers (5 blocks of 492000 cells: 112 / 145
+//    / 134 against 133 / 149 / 151 staged), or of 128 for fewer than eight waves (5
+//    blocks of 132000 cells: 29 / 45 / 45 against 45 / 58 / 58);
 //  - air: plane kernels of 80 registers (157 x 99 x 67: 114 / 131 / 143 against 165 /
 //    323 / 287, staged 139 / 147 / 148; Roe 147 / 173 / 182 against 220 / 444 / 393);
-//    a grid of one wave is latency-bound and takes 128 registers (41 x 33 x 10: 28
-//    against 32 for the three sweeps);
 //  - AWENO (no staged build, 240 registers wanted) and the rest: plane kernels of 128
-//    registers (128 x 96 x 80: 219 / 203 / 198 against 295 / 372 / 315).
+//    registers (128 x 96 x 80: 219 / 203 / 198 against 295 / 372 / 315);
+//  - a grid whose plane CTAs are all resident with 255 registers (two of 4 rows per
+//    SM, or one of 8) takes those: a smaller budget adds no CTA and costs spills
+//    (41 x 33 x 10 AWENO 31 against 37 for the three sweeps, Roe 32 against 35;
+//    16 x 16 x 16 Roe with 9 species 64 against 74; air with SST 31 x 25 x 21 32
+//    against 37 staged).
 // Rows and chunks: a CTA takes about C + 0.15 chunk times (0.15: start-up and the
 // carried face), so the pair with the fewest waves times that wins.
 void default_tiles(ostc_ctx *c) {
@@ -799,6 +806,9 @@ void default_tiles(ostc_ctx *c) {
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const bool aweno = c->prm.inviscid_type == 1, roe = c->prm.inviscid_type == 2;
   const bool viscous = c->prm.viscous_scheme != 0;
+  const bool air = c->ns == 0 && c->nt == 0, air_sst = c->ns == 0 && c->nt > 0;
+  bool even = false, odd = false;  // zones whose rows move by bulk copies, and others
+  for (const DevZone &z : c->dz) ((z.flags & kZoneBulk) ? even : odd) = true;
   for (int d = 0; d < 3; ++d) {
     auto tiles = [&](int R, int C) {
       long long n = 0;
@@ -809,20 +819,28 @@ void default_tiles(ostc_ctx *c) {
       return n;
     };
     const size_t smem = stage_smem_bytes(c->ns, c->nt, d, viscous) + 64 * (5 + c->ns + c->nt) + 1024;
-    const bool staged = !aweno && ((c->ns > 0 && !roe) || c->nt > 0) && 2 * smem <= 228 * 1024;
-    const bool air80 = !aweno && c->ns == 0 && c->nt == 0 && tiles(8, 1) > 2 * sms;
+    const bool staged = !aweno && ((c->ns > 0 && !roe) || c->nt > 0) && 2 * smem <= 228 * 1024 &&
+                        !(air_sst && even && odd);
+    if (!staged || air_sst) {
+      const int rows = tiles(4, 1) <= 2 * sms ? 4 : (tiles(8, 1) <= sms ? 8 : 0);
+      if (rows) {
+        c->tile[d] = TileShape{rows, 1, 1};
+        continue;
+      }
+    }
+    const bool r80 = !aweno && !staged && ((air && tiles(8, 1) > 2 * sms) || (air_sst && tiles(8, 1) > 8 * 2 * sms));
     TileShape best;
     double cost = -1;
     for (int R : {8, 4})
       for (int C : {1, 2}) {
         // staged CTAs have 8 rows, the 80-register plane CTAs 4; a 128-register CTA of one
         // wave takes 8
-        if (R == 4 ? staged : air80) continue;
-        const long long slots = (long long)sms * (air80 ? 6 : (R == 8 ? 2 : 4));
+        if (R == 4 ? staged : r80) continue;
+        const long long slots = (long long)sms * (r80 ? 6 : (R == 8 ? 2 : 4));
         const double w = (double)((tiles(R, C) + slots - 1) / slots) * (C + 0.15);
         if (cost < 0 || w < cost) {
           cost = w;
-          best = TileShape{R, C, air80 ? 3 : 2};
+          best = TileShape{R, C, r80 ? 3 : 2};
           best.staged = staged;
         }
       }
