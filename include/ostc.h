@@ -609,20 +609,37 @@ ostc_status ostc_autotune(ostc_ctx *ctx, int warmup, int reps, void *stream, flo
  * the last earlier face whose footprint meets its own: for interfaces own
  * range and plane, partner's range and plane), with a grid barrier between
  * waves, so the results are the per-face ones bit for bit. A barrier wait is
- * bounded (about one second); one that runs out makes the next check of a
- * call with histories return OSTC_ERR_TIMEOUT. At most 64 blocks:
+ * bounded (about one second); one that runs out is reported as
+ * OSTC_ERR_TIMEOUT (ostc_check). At most 64 blocks:
  * OSTC_ERR_UNSUPPORTED beyond. No reference counterpart: the reference
  * launches every kernel per block and face (RK.cuh:107-161).              */
 ostc_status ostc_set_batching(ostc_ctx *ctx, int on);
 ostc_status ostc_get_batching(const ostc_ctx *ctx, int *on);
 /* Diagnostic for failure handling: with on = 1 the grid barriers of the
  * batched boundary-face and interface launches withhold their release, so
- * each launch with more than one wave waits about one second, stops, and
- * the next ostc_rk3_steps / ostc_steady_steps with histories returns
- * OSTC_ERR_TIMEOUT (the waves after the first were not computed); on = 0
+ * each launch with more than one wave waits about one second, stops and is
+ * reported as OSTC_ERR_TIMEOUT (ostc_check; the waves after the first were
+ * not computed); on = 0
  * restores normal operation. Synchronises the device. No reference
  * counterpart.                                                              */
 ostc_status ostc_inject_wave_timeout(ostc_ctx *ctx, int on);
+/* The same for the staged flux kernels: with on = 1 the tiles that move as
+ * bulk copies (even row lengths) withhold their arrival, so that each CTA
+ * waits about two seconds and leaves its faces out. Drops the captured steps.
+ * Synchronises the device. No reference counterpart.                       */
+ostc_status ostc_inject_tile_timeout(ostc_ctx *ctx, int on);
+
+/* Waits for the stream, then returns OSTC_ERR_TIMEOUT when a bounded device
+ * wait of a kernel that this context launched has run out since the last
+ * report, and OSTC_OK otherwise. Such a wait (the tiles of the staged flux
+ * kernels, the grid barrier of the batched boundary faces and interfaces, the
+ * network of chem_mode 2) ends by itself after about a second and leaves work
+ * undone: the results since then are not valid. Calls that launch work do
+ * not wait for it, so they report an earlier call's wait, once, before they
+ * launch anything; calls that synchronise (ostc_global_time_step with
+ * dt_host, steps with histories) report their own. A host that reads results
+ * of other calls asks here first. No reference counterpart.                */
+ostc_status ostc_check(ostc_ctx *ctx, void *stream);
 
 /* Launch one kernel family on every block (timing and autotuning aid):
  * OSTC_OP_FLUX (arg = direction, accumulates into dq; arg + 3: the inviscid

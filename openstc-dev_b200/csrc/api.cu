@@ -88,6 +88,9 @@ struct ostc_ctx {
   double *chem_buf = nullptr;
   long long *chem_stats = nullptr;
   long long max_cells = 0;
+  // set by a kernel of this context whose bounded wait ran out (mapped host memory, so
+  // that the host reads it without a copy or a synchronisation)
+  int *late = nullptr;
   ostc_status last = OSTC_OK;
   int last_cuda = 0;
   int err_block = -1, err_i = 0, err_j = 0, err_k = 0, err_step = -1;
@@ -111,12 +114,23 @@ ostc_status fail(ostc_ctx *c, ostc_status s, cudaError_t e = cudaSuccess) {
     if (e_ != cudaSuccess) return fail(ctx, OSTC_ERR_CUDA, e_); \
   } while (0)
 
-// the run parameters and zone table of ctx in every kernel unit's constant
+// OSTC_ERR_TIMEOUT, once, when a bounded wait of a kernel that ctx launched has run out
+// since the last report. Work may still be running on the context's streams: what it
+// leaves undone is reported by a later call.
+ostc_status take_late(ostc_ctx *ctx) {
+  return __atomic_load_n(ctx->late, __ATOMIC_RELAXED) && __atomic_exchange_n(ctx->late, 0, __ATOMIC_ACQ_REL)
+             ? fail(ctx, OSTC_ERR_TIMEOUT)
+             : OSTC_OK;
+}
+
+// the start of a call that launches work: a wait of an earlier launch that ran out is
+// reported, then the run parameters and zone table of ctx are in every kernel unit's constant
 // memory, uploaded when another context (or none) was the last one uploaded.
 // Not inside a stream capture: an upload captured into a graph would happen
 // only when the graph runs, while later calls took it as done (ensure_graph
 // uploads before it captures).
 ostc_status ensure_param(ostc_ctx *ctx, cudaStream_t s) {
+  if (ostc_status st = take_late(ctx)) return st;
   if (g_uploaded != ctx) {
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     CK(cudaStreamIsCapturing(s, &cap));
@@ -397,7 +411,9 @@ ostc_status build_tables(ostc_ctx *ctx) {
   if (ctx->if_plan.n_waves) ctx->if_plan.ends = ctx->wave_ends_dev + ctx->bc_plan.n_waves;
   if (!ctx->wave_sync) {
     CK(cudaMalloc(&ctx->wave_sync, 2 * sizeof(WaveSync)));
-    CK(cudaMemset(ctx->wave_sync, 0, 2 * sizeof(WaveSync)));
+    WaveSync ws[2] = {};
+    ws[0].late = ws[1].late = ctx->dz[0].late;
+    CK(cudaMemcpy(ctx->wave_sync, ws, sizeof(ws), cudaMemcpyHostToDevice));
   }
   return OSTC_OK;
 }
@@ -571,6 +587,7 @@ void fill_devzone(const ostc_zone &z, DevZone &d) {
   d.bv_last = z.bv_last;
   d.isr = d.dq0 = d.dqk = d.lu = d.da = nullptr;
   d.piv = nullptr;
+  d.late = nullptr;
   d.tsj = z.turb_src_jac;
   d.jac = z.jac;
 }
@@ -903,8 +920,13 @@ ostc_status ostc_create(const ostc_config *cfg, const ostc_param *param, const o
   c->spec_mech = c->spec_ok;
   c->zones.assign(zones, zones + n_zones);
   c->dz.resize(n_zones);
+  CK(cudaHostAlloc((void **)&c->late, sizeof(int), cudaHostAllocMapped));
+  *c->late = 0;
+  int *late_dev = nullptr;
+  CK(cudaHostGetDevicePointer((void **)&late_dev, c->late, 0));
   for (int b = 0; b < n_zones; ++b) {
     fill_devzone(zones[b], c->dz[b]);
+    c->dz[b].late = late_dev;
     c->dz[b].block_id = b;
     double *soa = nullptr;
     CK(cudaMalloc(&soa, sizeof(double) * 9 * c->dz[b].sz));
@@ -1049,6 +1071,7 @@ ostc_status ostc_destroy(ostc_ctx *ctx) {
   cudaFree(ctx->ifaces_dev);
   cudaFree(ctx->wave_ends_dev);
   cudaFree(ctx->wave_sync);
+  cudaFreeHost(ctx->late);
   cudaFree(ctx->res_partial);
   cudaFree(ctx->hist_counter);
   cudaFree(ctx->bad_key);
@@ -1077,6 +1100,12 @@ ostc_status ostc_get_error(const ostc_ctx *ctx, int *cuda_error, int *block, int
   if (j) *j = ctx->err_j;
   if (k) *k = ctx->err_k;
   return ctx->last;
+}
+
+ostc_status ostc_check(ostc_ctx *ctx, void *stream) {
+  if (!ctx) return OSTC_ERR_INVALID_ARG;
+  CK(cudaStreamSynchronize(S(stream)));
+  return take_late(ctx);
 }
 
 const double *ostc_dt_device(const ostc_ctx *ctx) { return ctx ? (const double *)ctx->dt_bits : nullptr; }
@@ -1131,6 +1160,7 @@ ostc_status ostc_global_time_step(ostc_ctx *ctx, double *dt_host, void *stream) 
   if (dt_host) {
     CK(cudaMemcpyAsync(dt_host, ctx->dt_bits, sizeof(double), cudaMemcpyDeviceToHost, S(stream)));
     CK(cudaStreamSynchronize(S(stream)));
+    return take_late(ctx);
   }
   return OSTC_OK;
 }
@@ -1323,6 +1353,7 @@ static ostc_status enqueue_step(ostc_ctx *ctx, bool with_hist, cudaStream_t s) {
         ChemScratch w;
         CK(surrogate_scratch(ctx->sur, (int)n, &w));
         count = w.count;
+        w.err = z.late;  // no call reads the surrogate's own word after a step
         CK(launch_chem_surrogate<NS_SUR>(*surrogate_net(ctx->sur), (int)n, T, p, Y, dt, dY, dT, w, s));
       }
       CK(dispatch_ns(ctx->ns, [&](auto m) {
@@ -1410,27 +1441,12 @@ static ostc_status ensure_graph(ostc_ctx *ctx, bool hist, GraphEntry **out, bool
   return OSTC_OK;
 }
 
-// after a synchronised call with histories: the first non-physical cell found by
-// the residual epilogue, if any, becomes OSTC_ERR_NONPHYSICAL with its zone and
-// cell (ostc_get_error) and the step of the call it was found in (err_step)
+// after a synchronised call with histories: a wait that ran out (the steps are not
+// valid), else the first non-physical cell found by the residual epilogue, if any,
+// becomes OSTC_ERR_NONPHYSICAL with its zone and cell (ostc_get_error) and the step of
+// the call it was found in (err_step)
 static ostc_status check_state(ostc_ctx *ctx, unsigned long long key) {
-  // a staged flux kernel that gave up waiting for its tile (bounded wait) left
-  // its faces uncomputed: the steps are not valid
-  int late = 0;
-  CK(stage_timeouts(&late));
-  // likewise a wave launch whose grid barrier ran out (the waves after it
-  // were not computed); the flags are cleared for the next steps
-  if (ctx->wave_sync) {
-    WaveSync ws[2];
-    CK(cudaMemcpy(ws, ctx->wave_sync, sizeof(ws), cudaMemcpyDeviceToHost));
-    if (ws[0].timed_out || ws[1].timed_out) {
-      const int zero = 0;
-      for (int k = 0; k < 2; ++k)
-        CK(cudaMemcpy(&ctx->wave_sync[k].timed_out, &zero, sizeof(int), cudaMemcpyHostToDevice));
-      late = 1;
-    }
-  }
-  if (late) return fail(ctx, OSTC_ERR_TIMEOUT);
+  if (ostc_status st = take_late(ctx)) return st;
   if (key == ~0ull) return OSTC_OK;
   const long long q = (long long)(key & ((1ull << 34) - 1));
   const int b = (int)((key >> 34) & 1023);
@@ -1960,6 +1976,15 @@ ostc_status ostc_inject_wave_timeout(ostc_ctx *ctx, int on) {
   if (!ctx->wave_sync) return OSTC_ERR_INVALID_ARG;  // no batched faces on this context
   CK(cudaDeviceSynchronize());
   for (int k = 0; k < 2; ++k) CK(cudaMemcpy(&ctx->wave_sync[k].hold, &on, sizeof(int), cudaMemcpyHostToDevice));
+  return OSTC_OK;
+}
+
+ostc_status ostc_inject_tile_timeout(ostc_ctx *ctx, int on) {
+  if (!ctx || (on != 0 && on != 1)) return OSTC_ERR_INVALID_ARG;
+  CK(cudaDeviceSynchronize());
+  for (auto &z : ctx->dz) z.flags = on ? z.flags | kZoneHold : z.flags & ~kZoneHold;
+  drop_graphs(ctx);
+  if (g_uploaded == ctx) g_uploaded = nullptr;  // the next launch uploads the zone table
   return OSTC_OK;
 }
 

@@ -85,9 +85,21 @@ struct DevZone {
   // pivots, DA divisors
   double *dq0, *dqk, *lu, *da;
   unsigned char *piv;
+  // the context's word in mapped host memory that a kernel sets when a bounded wait ran
+  // out (wait_ran_out)
+  int *late;
 };
 
-constexpr int kZoneBulk = 1;
+// bits of DevZone::flags; kZoneHold: a diagnostic, the staged flux kernels' bulk tiles
+// withhold their arrival, so that their bounded waits run out (ostc_inject_tile_timeout)
+constexpr int kZoneBulk = 1, kZoneHold = 2;
+
+// a bounded wait of this launch ran out and work was left undone: the context's
+// next call, or ostc_check, reports it (api.cu: take_late)
+__device__ __forceinline__ void wait_ran_out(int *late) {
+  *(volatile int *)late = 1;
+  __threadfence_system();
+}
 
 __device__ __forceinline__ int gidx(const DevZone &z, int i, int j, int k) {
   return k * z.d1 + j * z.d2 + i + z.dt_;

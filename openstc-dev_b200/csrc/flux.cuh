@@ -271,22 +271,6 @@ __device__ __forceinline__ bool stage_bar_wait(unsigned bar, unsigned parity) {
   }
 }
 
-// set when a staged flux CTA gave up waiting for its tile (read and cleared
-// by the unit's host accessor, stage_timeout_read)
-static __device__ int g_stage_timeout;
-
-// host side: this unit's timeout flag, cleared after the read
-static cudaError_t stage_timeout_read(int *flag) {
-  int v = 0;
-  cudaError_t e = cudaMemcpyFromSymbol(&v, g_stage_timeout, sizeof(int));
-  if (e == cudaSuccess && v) {
-    const int zero = 0;
-    e = cudaMemcpyToSymbol(g_stage_timeout, &zero, sizeof(int));
-  }
-  *flag = v;
-  return e;
-}
-
 // base pointer of plane p of the cell tile (StagedPlanes order)
 template <int NT>
 __device__ __forceinline__ const double *stage_q_plane(const DevZone &z, int p) {
@@ -439,11 +423,11 @@ __device__ __forceinline__ bool flux_tile_staged(const DevZone &z, const int bx,
     stage_wait_all();
     if constexpr (BULK) {
       __syncthreads();  // every copying thread has announced its bytes
-      if (threadIdx.x == 0 && threadIdx.y == 0) stage_arrive(bar);
+      if (threadIdx.x == 0 && threadIdx.y == 0 && !(z.flags & kZoneHold)) stage_arrive(bar);
       const bool late = !stage_bar_wait(bar, phase);
       if (__syncthreads_or(late)) {
         // give up: record it, let the copies in flight land (bounded) and stop
-        if (threadIdx.x == 0 && threadIdx.y == 0) atomicExch(&g_stage_timeout, 1);
+        if (threadIdx.x == 0 && threadIdx.y == 0) wait_ran_out(z.late);
         stage_bar_wait(bar, phase);
         return false;
       }

@@ -926,8 +926,8 @@ __global__ void interface_kernel(DevZone z, DevZone t, Iface f, int with_cv) {
 // all CTAs have finished wave w, so wave w + 1 reads what wave w wrote. The
 // barrier counts arrivals in the context's WaveSync. Each wait is bounded by
 // the global timer: a CTA whose wait runs out sets abort (every other wait
-// then ends at once) and timed_out, which the host reads after the step; the
-// waves after it are not computed. The last CTA to leave resets the counters
+// then ends at once) and the context's word that reports it; the waves after
+// it are not computed. The last CTA to leave resets the counters
 // for the next launch on the stream.
 // ---------------------------------------------------------------------------
 constexpr unsigned long long kWaveWaitNs = 1000000000ull;  // 1 s
@@ -953,7 +953,7 @@ __device__ __forceinline__ bool wave_barrier(WaveSync *s, unsigned target) {
     }
     if (*(volatile int *)&s->abort) return false;
     if ((it & 15) == 15 && wave_clock() - t0 > kWaveWaitNs) {
-      atomicExch(&s->timed_out, 1);
+      wait_ran_out(s->late);
       atomicExch(&s->abort, 1);
       return false;
     }
@@ -1521,21 +1521,6 @@ bool mechanism_is_h2air9(const int *reac_type, const int *stoi_f, const int *sto
         return false;
   }
   return true;
-}
-
-// any staged-flux tile wait that ran out, over all flux units (flags cleared)
-cudaError_t stage_timeouts(int *any) {
-  cudaError_t (*const fns[])(int *) = {stage_timeout_flux0,     stage_timeout_flux9,     stage_timeout_flux0t,
-                                        stage_timeout_flux9t,    stage_timeout_flux_ns_a, stage_timeout_flux_ns_b,
-                                        stage_timeout_flux_ns_c, stage_timeout_flux_ns_d};
-  *any = 0;
-  for (auto fn : fns) {
-    int f = 0;
-    const cudaError_t e = fn(&f);
-    if (e != cudaSuccess) return e;
-    *any |= f;
-  }
-  return cudaSuccess;
 }
 
 // this unit's parameters and those of the units that ns species and nt turbulence

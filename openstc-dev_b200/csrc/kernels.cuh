@@ -126,15 +126,6 @@ cudaError_t upload_zones_flux0t(const DevZone *z, int n, cudaStream_t s);  // fl
 cudaError_t upload_zones_flux9t(const DevZone *z, int n, cudaStream_t s);  // flux9t.cu
 // staged flux kernels: whether a tile wait ran out since the last read (the
 // flag is cleared), per flux unit and over all of them (kernels.cu)
-cudaError_t stage_timeout_flux0(int *flag);
-cudaError_t stage_timeout_flux9(int *flag);
-cudaError_t stage_timeout_flux0t(int *flag);
-cudaError_t stage_timeout_flux9t(int *flag);
-cudaError_t stage_timeout_flux_ns_a(int *flag);
-cudaError_t stage_timeout_flux_ns_b(int *flag);
-cudaError_t stage_timeout_flux_ns_c(int *flag);
-cudaError_t stage_timeout_flux_ns_d(int *flag);
-cudaError_t stage_timeouts(int *any);
 template <int NS>
 cudaError_t launch_bc(const DevZone &z, const BcFace &b, int with_cv, cudaStream_t s);
 // The waves of one call (boundary faces or interfaces over every zone; device
@@ -151,12 +142,13 @@ struct WavePlan {
 };
 // the grid barrier of a wave launch (device memory of the context, zeroed
 // once): arrivals, CTAs that have left, the abort flag of a wait that ran
-// out, timed_out, which stays set until the host reads and clears it, and
-// hold, a diagnostic the host sets to withhold every barrier's release (its
-// waits then run out: ostc_inject_wave_timeout)
+// out, hold, a diagnostic the host sets to withhold every barrier's release
+// (its waits then run out: ostc_inject_wave_timeout), and the context's word
+// that reports such a wait (DevZone::late)
 struct WaveSync {
   unsigned arrive, done;
-  int abort, timed_out, hold, pad;
+  int abort, hold;
+  int *late;
 };
 template <int NS>
 cudaError_t launch_bc_waves(const BcFace *faces, const WavePlan &p, int with_cv, WaveSync *sync, cudaStream_t s);

@@ -136,6 +136,8 @@ def lib():
             "ostc_set_batching": [vp, i],
             "ostc_get_batching": [vp, C.POINTER(i)],
             "ostc_inject_wave_timeout": [vp, i],
+            "ostc_inject_tile_timeout": [vp, i],
+            "ostc_check": [vp, vp],
             "ostc_launch_op": [vp, i, i, vp],
             "ostc_autotune": [vp, i, i, vp, C.POINTER(C.c_float)],
             "ostc_set_interfaces": [vp, C.POINTER(IfaceC), i],
@@ -725,9 +727,19 @@ class Solver:
 
     def inject_wave_timeout(self, on: bool):
         """diagnostic: make the grid barriers of the batched boundary-face and
-        interface launches run out (calls with histories then return
-        OSTC_ERR_TIMEOUT)"""
+        interface launches run out (reported as OSTC_ERR_TIMEOUT)"""
         check(lib().ostc_inject_wave_timeout(self.ctx, 1 if on else 0), "ostc_inject_wave_timeout")
+
+    def inject_tile_timeout(self, on: bool):
+        """diagnostic: make the tile waits of the staged flux kernels run out
+        (reported as OSTC_ERR_TIMEOUT)"""
+        check(lib().ostc_inject_tile_timeout(self.ctx, 1 if on else 0), "ostc_inject_tile_timeout")
+
+    def check(self):
+        """waits for the current stream and raises OstcError when a bounded device
+        wait of this solver's launches has run out since the last report (results
+        are then not valid); steps with histories report it by themselves"""
+        check(lib().ostc_check(self.ctx, self._s()), "ostc_check")
 
     def batching(self) -> bool:
         v = C.c_int()

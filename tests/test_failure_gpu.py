@@ -11,7 +11,11 @@
 * likewise the bounded grid barrier between the waves of the batched
   boundary-face and interface launches (its release withheld on request):
   the steps with histories return OSTC_ERR_TIMEOUT and, with the release
-  restored, the same context steps as a fresh one.
+  restored, the same context steps as a fresh one;
+* calls that do not synchronise (a residual, boundary conditions, steps
+  without histories) leave their report to the context's next call or to
+  ostc_check, never to another context; the staged sweeps' tile waits (arrival
+  withheld) and the network's inside the split step are reported alike.
 """
 import time
 
@@ -122,3 +126,72 @@ def test_bounded_wave_barrier_runs_out_and_recovers():
     res, dts = s.rk3_steps(2, history=True)
     assert np.array_equal(res, res_ref) and np.array_equal(dts, dt_ref)
     s.close()
+
+
+def _timeout(call, *a, **k):
+    with pytest.raises(ostc.OstcError) as e:
+        call(*a, **k)
+    assert e.value.status == ostc.ERR_TIMEOUT
+
+
+def test_tile_wait_of_a_residual_is_reported():
+    case = ostc.case_mixing_layer(32, 30, 8)
+    s, blocks = case.solver()
+    assert s.get_tile(0)[0] >> 16 == 1  # staged by default, and even rows move by bulk copies
+    other, _ = ostc.case_mixing_layer(16, 14, 8).solver()
+    s.initialize()
+    other.initialize()
+    s.compute_rhs()
+    s.check()
+    ref = blocks[0].download("dq").copy()
+    s.inject_tile_timeout(True)
+    t0 = time.perf_counter()
+    s.compute_rhs()
+    _timeout(s.check)
+    assert 0.5 < time.perf_counter() - t0 < 60.0
+    s.check()  # reported once
+    s.launch_op(s.OP_FLUX, 0)
+    other.check()
+    assert np.isfinite(other.rk3_steps(1, history=True)[0]).all()  # not the other context's
+    s.inject_tile_timeout(False)
+    _timeout(s.compute_rhs)  # the launch above, reported by the next call
+    s.compute_rhs()
+    s.check()
+    assert np.array_equal(blocks[0].download("dq"), ref)
+    s.close()
+    other.close()
+
+
+def test_wave_wait_without_histories_is_reported():
+    s, blocks = ostc.case_uneven_blocks(
+        layout=ostc.block_layout(5, dims=(40, 30, 32), ranges=((8, 20), (8, 14), (8, 10)), anchors=False)).solver()
+    s.initialize()
+    s.rk3_steps(1)
+    s.check()
+    s.inject_wave_timeout(True)
+    s.apply_boundary_conditions(True)
+    _timeout(s.check)
+    s.rk3_steps(1)
+    _timeout(s.check)
+    s.apply_boundary_conditions(True)
+    s.inject_wave_timeout(False)  # (synchronises)
+    _timeout(s.rk3_steps, 1)
+    s.rk3_steps(1)
+    s.check()
+    s.close()
+
+
+def test_network_wait_of_a_split_step_is_reported():
+    case = ostc.case_premixed_box(16, 14, 8, dx=1e-3, T0=1500.0)
+    case.scheme.chem_mode = 2
+    s, _ = case.solver()
+    sur = ostc.Surrogate(max_batch=1024, seed=3)
+    sur.set_checks(np.ones((1, 9)), np.ones(1), 0.0, 0.0)  # every state to the FP64 integrator
+    sur.inject_timeout(True)
+    s.set_chem_surrogate(sur)
+    s.initialize()
+    _timeout(s.rk3_steps, 1, history=True)
+    s.rk3_steps(1)
+    _timeout(s.check)
+    s.close()
+    sur.close()
