@@ -519,7 +519,7 @@ __device__ __forceinline__ unsigned stage_bar_setup(unsigned long long *bar_mem)
 
 // BULK: every zone the launch walks has kZoneBulk (the launcher checks)
 template <int NS, int INV, int DIR, int MINB, int PART, int NT, bool BULK>
-__global__ void __launch_bounds__(FluxBounds<MINB>::threads, FluxBounds<MINB>::blocks)
+static __global__ void __launch_bounds__(FluxBounds<MINB>::threads, FluxBounds<MINB>::blocks)
     flux_dir_staged(DevZone z, int nchunk, int accumulate, int viscous) {
   extern __shared__ __align__(16) double smem[];
   __shared__ unsigned long long bar_mem;
@@ -530,7 +530,7 @@ __global__ void __launch_bounds__(FluxBounds<MINB>::threads, FluxBounds<MINB>::b
 }
 
 template <int NS, int INV, int DIR, int MINB, int PART, int NT, bool BULK>
-__global__ void __launch_bounds__(FluxBounds<MINB>::threads, FluxBounds<MINB>::blocks)
+static __global__ void __launch_bounds__(FluxBounds<MINB>::threads, FluxBounds<MINB>::blocks)
     flux_dir_staged_table(const int4 *tiles, int n_tiles, int nchunk, int accumulate, int viscous) {
   extern __shared__ __align__(16) double smem[];
   __shared__ unsigned long long bar_mem;
@@ -545,7 +545,7 @@ __global__ void __launch_bounds__(FluxBounds<MINB>::threads, FluxBounds<MINB>::b
 }
 
 template <int NS, int INV, int DIR, int MINB, int PART, int NT>
-__global__ void __launch_bounds__(FluxBounds<MINB>::threads, FluxBounds<MINB>::blocks)
+static __global__ void __launch_bounds__(FluxBounds<MINB>::threads, FluxBounds<MINB>::blocks)
     flux_dir(DevZone z, int nchunk, int accumulate, int viscous) {
   flux_tile<NS, INV, DIR, PART, NT>(z, blockIdx.x, blockIdx.y, blockIdx.z, nchunk, accumulate, viscous);
 }
@@ -553,7 +553,7 @@ __global__ void __launch_bounds__(FluxBounds<MINB>::threads, FluxBounds<MINB>::b
 // all zones of the context in one launch: a persistent grid walks the tile
 // table of {zone, bx, by, bz} segments (zones in c_zones)
 template <int NS, int INV, int DIR, int MINB, int PART, int NT>
-__global__ void __launch_bounds__(FluxBounds<MINB>::threads, FluxBounds<MINB>::blocks)
+static __global__ void __launch_bounds__(FluxBounds<MINB>::threads, FluxBounds<MINB>::blocks)
     flux_dir_table(const int4 *tiles, int n_tiles, int nchunk, int accumulate, int viscous) {
   for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
     const int4 c = tiles[t];

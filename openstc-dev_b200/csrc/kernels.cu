@@ -77,7 +77,7 @@ __device__ __forceinline__ void source_cells(const DevZone &z, const int bx, con
 }
 
 template <int NS, int SPEC>
-__global__ void __launch_bounds__(256) source_kernel(DevZone z) {
+static __global__ void __launch_bounds__(256) source_kernel(DevZone z) {
   source_cells<NS, SPEC>(z, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
@@ -85,7 +85,7 @@ __global__ void __launch_bounds__(256) source_kernel(DevZone z) {
 // batched FP64 point-implicit chemistry integrator (point_implicit_increment)
 // over n states held as SoA device arrays: Y and dY are [NS][n]
 template <int NS>
-__global__ void __launch_bounds__(128) chem_integrator_kernel(int n, const double *T, const double *p, const double *Y,
+static __global__ void __launch_bounds__(128) chem_integrator_kernel(int n, const double *T, const double *p, const double *Y,
                                                               const double *dt, double *dY, double *dT) {
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q >= n) return;
@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(128) chem_integrator_kernel(int n, const doubl
 // arrays (T, p, Y [NS][n], dt), and scatter the increments back at constant
 // density and internal energy (Y, T, p, the species cv; rho E unchanged)
 template <int NS>
-__global__ void __launch_bounds__(256) chem_gather_kernel(DevZone z, const double *dt_dev, double dt_fixed, double *T,
+static __global__ void __launch_bounds__(256) chem_gather_kernel(DevZone z, const double *dt_dev, double dt_fixed, double *T,
                                                           double *p, double *Y, double *dt) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(256) chem_gather_kernel(DevZone z, const doubl
 }
 
 template <int NS>
-__global__ void __launch_bounds__(256) chem_scatter_kernel(DevZone z, const double *dY, const double *dT) {
+static __global__ void __launch_bounds__(256) chem_scatter_kernel(DevZone z, const double *dY, const double *dT) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y;
   const int k = blockIdx.z;
@@ -228,7 +228,7 @@ __device__ __forceinline__ void update_rk_cells(const DevZone &z, const int bx, 
 }
 
 template <int NS>
-__global__ void __launch_bounds__(256) update_rk_kernel(DevZone z, double dt_in, const double *dt_dev, int rk) {
+static __global__ void __launch_bounds__(256) update_rk_kernel(DevZone z, double dt_in, const double *dt_dev, int rk) {
   update_rk_cells<NS>(z, blockIdx.x, blockIdx.y, blockIdx.z, dt_in, dt_dev, rk);
 }
 
@@ -276,7 +276,7 @@ __device__ __forceinline__ void properties_cells(const DevZone &z, const int bx,
 }
 
 template <int NS>
-__global__ void __launch_bounds__(256) properties_kernel(DevZone z) {
+static __global__ void __launch_bounds__(256) properties_kernel(DevZone z) {
   properties_cells<NS>(z, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
@@ -304,7 +304,7 @@ __device__ __forceinline__ void init_mut_cells(const DevZone &z, const int bx, c
 }
 
 template <int NS>
-__global__ void __launch_bounds__(256) init_mut_kernel(DevZone z) {
+static __global__ void __launch_bounds__(256) init_mut_kernel(DevZone z) {
   init_mut_cells<NS>(z, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
@@ -348,7 +348,7 @@ __device__ __forceinline__ void cv_from_bv_cells(const DevZone &z, const int bx,
 }
 
 template <int NS>
-__global__ void __launch_bounds__(256) cv_from_bv_kernel(DevZone z) {
+static __global__ void __launch_bounds__(256) cv_from_bv_kernel(DevZone z) {
   cv_from_bv_cells<NS>(z, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
@@ -423,7 +423,7 @@ __device__ __forceinline__ void dt_cells(const DevZone &z, const int bx, const i
 }
 
 template <int NS>
-__global__ void __launch_bounds__(256) dt_kernel(DevZone z, unsigned long long *dt_bits) {
+static __global__ void __launch_bounds__(256) dt_kernel(DevZone z, unsigned long long *dt_bits) {
   dt_cells<NS>(z, blockIdx.x, blockIdx.y, blockIdx.z, dt_bits);
 }
 
@@ -833,7 +833,7 @@ static __device__ __forceinline__ void bc_subsonic_inflow_point(const DevZone &z
 
 // per-face kernels: the launch of one face's points (launch_bc)
 #define OSTC_BC_KERNEL(name, point)                                      \
-  __global__ void name(DevZone z, BcFace b, int with_cv) {               \
+  static __global__ void name(DevZone z, BcFace b, int with_cv) {        \
     const int i = b.rs[0] + blockIdx.x * blockDim.x + threadIdx.x;       \
     const int j = b.rs[1] + blockIdx.y * blockDim.y + threadIdx.y;       \
     const int k = b.rs[2] + blockIdx.z;                                  \
@@ -854,7 +854,7 @@ template <int NS>
 OSTC_BC_KERNEL(bc_farfield_kernel, bc_farfield_point<NS>)
 template <int NS>
 OSTC_BC_KERNEL(bc_back_pressure_kernel, bc_back_pressure_point<NS>)
-static OSTC_BC_KERNEL(bc_subsonic_inflow_kernel, bc_subsonic_inflow_point)
+OSTC_BC_KERNEL(bc_subsonic_inflow_kernel, bc_subsonic_inflow_point)
 #undef OSTC_BC_KERNEL
 
 // one point of a boundary face of any type (the face records of the wave
@@ -910,7 +910,7 @@ __device__ __forceinline__ void interface_point(const DevZone &z, const DevZone 
 }
 
 template <int NS>
-__global__ void interface_kernel(DevZone z, DevZone t, Iface f, int with_cv) {
+static __global__ void interface_kernel(DevZone z, DevZone t, Iface f, int with_cv) {
   const int n0 = blockIdx.x * blockDim.x + threadIdx.x;
   const int n1 = blockIdx.y * blockDim.y + threadIdx.y;
   const int n2 = blockIdx.z;
@@ -962,7 +962,7 @@ __device__ __forceinline__ bool wave_barrier(WaveSync *s, unsigned target) {
 }
 
 template <int NS, int KIND>
-__global__ void __launch_bounds__(256) waves_kernel(const void *records, const int4 *tiles, const int *ends,
+static __global__ void __launch_bounds__(256) waves_kernel(const void *records, const int4 *tiles, const int *ends,
                                                     int n_waves, int with_cv, WaveSync *sync) {
   __shared__ int go_on;
   const bool lead = threadIdx.x == 0 && threadIdx.y == 0;
@@ -1107,7 +1107,7 @@ static __global__ void residual_final_kernel(const double *partial, int n_part, 
 // CTAs walks {zone, bx, by, bz} tiles of every zone (zones in c_zones)
 // ---------------------------------------------------------------------------
 template <class Op>
-__global__ void __launch_bounds__(256) cells_table_kernel(const int4 *tiles, int n_tiles, Op op) {
+static __global__ void __launch_bounds__(256) cells_table_kernel(const int4 *tiles, int n_tiles, Op op) {
   for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
     const int4 c = tiles[t];
     op(c_zones[c.x], c.y, c.z, c.w);
@@ -1135,8 +1135,6 @@ template <int NS>
 struct CvOp {
   __device__ void operator()(const DevZone &z, int bx, int by, int bz) const { cv_from_bv_cells<NS>(z, bx, by, bz); }
 };
-// (every Op carries its species count: a kernel of the same name in two units would be
-// one symbol, and run with either unit's zone table)
 template <int NS>
 struct VelocityOp {
   __device__ void operator()(const DevZone &z, int bx, int by, int bz) const { velocity_cells(z, bx, by, bz); }
@@ -1188,7 +1186,10 @@ cudaError_t launch_table(const CellTable &tab, const Op &op, cudaStream_t s) {
 
 #ifndef OSTC_NS_UNIT
 // the kernel units a context of ns species and nt turbulence scalars launches, besides
-// this one: its sweeps' and, for counts other than 0 and 9, its per-cell kernels'
+// this one: its sweeps' and, for counts other than 0 and 9, its per-cell kernels'. A unit's
+// kernels read the unit's own copies, which only its contexts write: every kernel of a file
+// that several units compile is static, since of a template that two units instantiate with
+// external linkage the linker keeps one, and it would run with that unit's copies.
 struct UnitUploads {
   cudaError_t (*param[2])(const DevParam &, cudaStream_t);
   cudaError_t (*zones[2])(const DevZone *, int, cudaStream_t);

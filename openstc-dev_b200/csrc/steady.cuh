@@ -440,26 +440,26 @@ __device__ __forceinline__ void dplur_finish_cells(const DevZone &z, const int b
 
 // one zone's launch of each
 template <int NS, int SPEC>
-__global__ void __launch_bounds__(128) chem_implicit_kernel(DevZone z) {
+static __global__ void __launch_bounds__(128) chem_implicit_kernel(DevZone z) {
   chem_implicit_cells<NS, SPEC>(z, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 template <int NS>
-__global__ void __launch_bounds__(256) update_bv_kernel(DevZone z) {
+static __global__ void __launch_bounds__(256) update_bv_kernel(DevZone z) {
   update_bv_cells<NS>(z, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 static __global__ void __launch_bounds__(256) turb_implicit_kernel(DevZone z) {
   turb_implicit_cells(z, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 template <int NS, int SPEC>
-__global__ void __launch_bounds__(128) dplur_dq0_kernel(DevZone z, SteadyArgs a) {
+static __global__ void __launch_bounds__(128) dplur_dq0_kernel(DevZone z, SteadyArgs a) {
   dplur_dq0_cells<NS, SPEC>(z, blockIdx.x, blockIdx.y, blockIdx.z, a);
 }
 template <int NS, int SPEC>
-__global__ void __launch_bounds__(128) dplur_sweep_kernel(DevZone z, SteadyArgs a) {
+static __global__ void __launch_bounds__(128) dplur_sweep_kernel(DevZone z, SteadyArgs a) {
   dplur_sweep_cells<NS, SPEC>(z, blockIdx.x, blockIdx.y, blockIdx.z, a);
 }
 template <int NS>
-__global__ void __launch_bounds__(256) dplur_finish_kernel(DevZone z) {
+static __global__ void __launch_bounds__(256) dplur_finish_kernel(DevZone z) {
   dplur_finish_cells<NS>(z, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 

@@ -118,7 +118,7 @@ __device__ void fill_chem_tables(ChemTables<NS> *t, const double *scale, const m
 // features, the training-envelope test, and the standardised features as a
 // BF16 row of the network's first operand (12 features, 4 zeros)
 template <int NS>
-__global__ void __launch_bounds__(256) chem_features_kernel(int n, const double *T, const double *p, const double *Y,
+static __global__ void __launch_bounds__(256) chem_features_kernel(int n, const double *T, const double *p, const double *Y,
                                                             const double *dt, const double *scale,
                                                             const mlp::Checks *ck, __nv_bfloat16 *x,
                                                             unsigned char *env) {
@@ -159,7 +159,7 @@ static __global__ void __launch_bounds__(tc::THREADS, 1) surrogate_chem_kernel(m
 // the element-mass and internal-energy checks in FP32; a state outside the
 // envelope or failing a check goes to the fallback list (warp-aggregated)
 template <int NS>
-__global__ void __launch_bounds__(256, 3) chem_checks_kernel(int n, const double *T, const double *Y, const double *dt,
+static __global__ void __launch_bounds__(256, 3) chem_checks_kernel(int n, const double *T, const double *Y, const double *dt,
                                                           const float *y, const unsigned char *env,
                                                           const double *scale, const mlp::Checks *ck, double *dY,
                                                           double *dT, int *list, int *count) {
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(256, 3) chem_checks_kernel(int n, const double
 }
 
 template <int NS>
-__global__ void __launch_bounds__(128) chem_fallback_kernel(const int *list, const int *count, int n, const double *T,
+static __global__ void __launch_bounds__(128) chem_fallback_kernel(const int *list, const int *count, int n, const double *T,
                                                             const double *p, const double *Y, const double *dt,
                                                             double *dY, double *dT) {
   if constexpr (NS > 0) {
