@@ -631,7 +631,9 @@ static cudaError_t launch_flux_sb(const DevZone &z, const TileShape &t, const Fl
   if (t.rows != SR) return cudaErrorInvalidConfiguration;
   const bool vis_planes = PART == 2 || (PART == 0 && viscous);
   const size_t smem = sizeof(double) * stage_smem_doubles<NS, NT, DIR>(vis_planes);
-  if (smem != stage_smem_bytes(NS, NT, DIR, vis_planes)) return cudaErrorInvalidConfiguration;
+  static_assert(sizeof(double) * stage_smem_doubles<NS, NT, DIR>(false) == stage_smem_bytes(NS, NT, DIR, false) &&
+                    sizeof(double) * stage_smem_doubles<NS, NT, DIR>(true) == stage_smem_bytes(NS, NT, DIR, true),
+                "default_tiles chooses by this kernel's shared memory");
   if (smem > 227 * 1024) return cudaErrorInvalidConfiguration;
   const void *fn = tab ? (const void *)flux_dir_staged_table<NS, INV, DIR, MINB, PART, NT, BULK>
                        : (const void *)flux_dir_staged<NS, INV, DIR, MINB, PART, NT, BULK>;

@@ -47,8 +47,9 @@ inline dim3 flux_grid(int mx, int my, int mz, int dir, int R, int C) {
   return dim3((mx + 31) / 32, my, (mz + S - 1) / S);
 }
 
-// dynamic shared memory (bytes) of a staged flux CTA (flux.cuh: stage_smem_doubles)
-inline size_t stage_smem_bytes(int ns, int nt, int dir, bool viscous) {
+// dynamic shared memory (bytes) of a staged flux CTA, for the choice of default tiles; the
+// staged launchers assert that it is their own (flux.cuh: stage_smem_doubles)
+constexpr size_t stage_smem_bytes(int ns, int nt, int dir, bool viscous) {
   const size_t tv = (dir == 0 ? 10 : 11) * 36, qv = (dir == 0 ? 8 : 9) * 34;
   const size_t nq = viscous ? (nt > 0 ? 15 : 12) + ns : 10;
   return sizeof(double) * ((6 + ns + nt) * tv + nq * qv + (dir == 0 ? 0 : (5 + ns + nt) * 32));
