@@ -1642,11 +1642,11 @@ ostc_status ostc_chem_surrogate(ostc_ctx *ctx, ostc_surrogate *sur, int n, const
   CK(prepare_chem_surrogate());
   ChemScratch w;
   CK(surrogate_scratch(sur, n > 0 ? n : 1, &w));
-  CK(cudaMemsetAsync(w.err, 0, sizeof(int), S(stream)));
+  CK(cudaMemsetAsync(w.count, 0, 2 * sizeof(int), S(stream)));  // count, err (mlp.cuh): read below for n = 0 too
   CK(launch_chem_surrogate<mlp::NIN - 3>(*surrogate_net(sur), n, T, p, Y, dt, dY, dT, w, S(stream)));
   if (n_fallback) {
     int h[2] = {0, 0};
-    CK(cudaMemcpyAsync(h, w.count, sizeof(h), cudaMemcpyDeviceToHost, S(stream)));  // count, err (mlp.cuh)
+    CK(cudaMemcpyAsync(h, w.count, sizeof(h), cudaMemcpyDeviceToHost, S(stream)));
     CK(cudaStreamSynchronize(S(stream)));
     *n_fallback = h[0];
     if (h[1]) return fail(ctx, OSTC_ERR_TIMEOUT);

@@ -179,3 +179,20 @@ def test_surrogate_gain_over_the_integrator(trained_on_runs):
     assert float(eT.max()) < 1.0 and float(eY.max()) < 1e-4
     assert ms["surrogate"] < ms["integrator"], ms
     s.close()
+
+
+def test_an_empty_batch_redoes_no_state():
+    """the count of redone states belongs to the call, also to one without states"""
+    import torch
+
+    case = _premixed(1)
+    s, _ = case.solver()
+    sur = ostc.Surrogate(max_batch=64, seed=3)
+    sur.set_checks(np.ones((1, 9)), np.ones(1), 0.0, 0.0)  # rejects every step
+    st = [torch.from_numpy(a).cuda() for a in ostc.sample_chem_states(case.mech, 50, seed=2)]
+    assert s.chem_surrogate(sur, *st)[2] == 50
+    none = [a[..., :0].contiguous() for a in st]
+    dY, dT, redone = s.chem_surrogate(sur, *none)
+    assert redone == 0 and dT.numel() == 0 and dY.numel() == 0
+    s.close()
+    sur.close()
