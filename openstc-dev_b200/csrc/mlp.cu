@@ -212,7 +212,8 @@ __global__ void loss_grad_kernel(const float *z4, const float *y, int n, float *
   if (threadIdx.x == 0) atomicAdd(loss_sum, red[0]);
 }
 
-// dZ = dA * silu'(Z) of a hidden layer: the BF16 copy, its transpose dzt [256][ldt] (the
+// dZ = dA * silu'(Z) of a hidden layer: the BF16 copy (null for the first, whose input
+// gradient nothing takes), its transpose dzt [256][ldt] (the
 // K-major operand of the weight gradient, zero from row n to ldt) and the bias gradient's
 // column sums (added into db, from the FP32 values). Bound by HBM: dA and Z in, two BF16
 // copies out. One CTA takes 64 columns of `rows` rows, 64 x 64 at a time: 16-byte loads,
@@ -243,7 +244,7 @@ __global__ void __launch_bounds__(256) silu_backward_kernel(const float *da, con
           d[e] = aa[e] * sg * (1.0f + zz[e] * (1.0f - sg));
           sum[e] += d[e];
         }
-        *(uint2 *)(dzb + o) = make_uint2(tc::pack_bf16(d[0], d[1]), tc::pack_bf16(d[2], d[3]));
+        if (dzb) *(uint2 *)(dzb + o) = make_uint2(tc::pack_bf16(d[0], d[1]), tc::pack_bf16(d[2], d[3]));
       }
 #pragma unroll
       for (int e = 0; e < 4; ++e) t[4 * cx + e][ry + 16 * i] = __float2bfloat16_rn(d[e]);
@@ -559,7 +560,7 @@ ostc_status ostc_surrogate_create(int max_batch, unsigned long long seed, ostc_s
   for (int l = 0; l < 4 && ok; ++l) {
     const long long w = l == 3 ? NOUTP : NH;
     ok = dalloc(s, (void **)&s->z[l], sizeof(float) * B * w) == cudaSuccess &&
-         dalloc(s, (void **)&s->dzb[l], sizeof(__nv_bfloat16) * B * w) == cudaSuccess;
+         (l == 0 || dalloc(s, (void **)&s->dzb[l], sizeof(__nv_bfloat16) * B * w) == cudaSuccess);
     if (ok && l < 3)
       ok = dalloc(s, (void **)&s->a[l], sizeof(__nv_bfloat16) * B * NH) == cudaSuccess &&
            dalloc(s, (void **)&s->ta[l + 1], sizeof(__nv_bfloat16) * NH * ((B + 15) / 16 * 16)) == cudaSuccess;
