@@ -813,9 +813,9 @@ void build_devparam(const ostc_param *p, DevParam &d) {
 //    registers (128 x 96 x 80: 219 / 203 / 198 against 295 / 372 / 315);
 //  - a grid whose plane CTAs are all resident with 255 registers (two of 4 rows per
 //    SM, or one of 8) takes those: a smaller budget adds no CTA and costs spills
-//    (41 x 33 x 10 AWENO 31 against 37 for the three sweeps, Roe 32 against 35;
-//    16 x 16 x 16 Roe with 9 species 64 against 74; air with SST 31 x 25 x 21 32
-//    against 37 staged).
+//    (residuals of 41 x 33 x 10 Roe 30.8 against 32.0, of 16 x 16 x 16 AWENO 28.7 against
+//    34.9 and Roe with nine species 88 against 95; the sweeps of 31 x 25 x 21 air with SST
+//    32 against 37 staged).
 // Rows and chunks: a CTA takes about C + 0.15 chunk times (0.15: start-up and the
 // carried face), so the pair with the fewest waves times that wins.
 void default_tiles(ostc_ctx *c) {
@@ -1984,7 +1984,6 @@ ostc_status ostc_inject_tile_timeout(ostc_ctx *ctx, int on) {
   CK(cudaDeviceSynchronize());
   for (auto &z : ctx->dz) z.flags = on ? z.flags | kZoneHold : z.flags & ~kZoneHold;
   drop_graphs(ctx);
-  if (g_uploaded == ctx) g_uploaded = nullptr;  // the next launch uploads the zone table
   return OSTC_OK;
 }
 

@@ -387,18 +387,20 @@ __device__ __forceinline__ void stage_issue(const DevZone &z, double *tile, doub
 
 // one segment (bx, by, bz) of zone z; BULK: the tiles move as bulk copies (the
 // zone has kZoneBulk), else as 8-byte cp.async; bar: the CTA's initialised tile
-// mbarrier, phase: its current phase parity (advanced per bulk chunk). Returns
-// false when a tile wait ran out (CTA-uniform; the kernel then stops).
+// mbarrier, phase: its current phase parity (advanced per bulk chunk); flags: bit 0
+// viscous faces, kZoneHold (a launch argument: read from the zone table, it cost a step
+// of SST blocks 1 %). Returns false when a tile wait ran out (CTA-uniform; the kernel
+// then stops).
 template <int NS, int INV, int DIR, int PART, int NT, bool BULK>
 __device__ __forceinline__ bool flux_tile_staged(const DevZone &z, const int bx, const int by, const int bz,
-                                                 int nchunk, int accumulate, int viscous, double *smem, unsigned bar,
+                                                 int nchunk, int accumulate, int flags, double *smem, unsigned bar,
                                                  unsigned &phase) {
   using Geo = StageGeom<DIR>;
   constexpr int NV = 5 + NS + NT, NVAR = 6 + NS + NT, R = SR;
   static_assert(INV != 1, "AWENO reads its cells (and the central correction's) from the planes");
   const int lane = threadIdx.x, row = threadIdx.y;
   const int n = DIR == 0 ? z.mx : (DIR == 1 ? z.my : z.mz);
-  const bool vis = viscous != 0;
+  const bool vis = (flags & 1) != 0;
   const int nq = stage_q_planes<NS, NT>(PART == 2 || (PART == 0 && vis));
   double *tile = smem;                                  // state tile; y / z: then the chunk's face fluxes
   double *qtile = smem + (size_t)NVAR * Geo::TV;        // cell tile
@@ -423,7 +425,7 @@ __device__ __forceinline__ bool flux_tile_staged(const DevZone &z, const int bx,
     stage_wait_all();
     if constexpr (BULK) {
       __syncthreads();  // every copying thread has announced its bytes
-      if (threadIdx.x == 0 && threadIdx.y == 0 && !(z.flags & kZoneHold)) stage_arrive(bar);
+      if (threadIdx.x == 0 && threadIdx.y == 0 && !(flags & kZoneHold)) stage_arrive(bar);
       const bool late = !stage_bar_wait(bar, phase);
       if (__syncthreads_or(late)) {
         // give up: record it, let the copies in flight land (bounded) and stop
@@ -520,25 +522,25 @@ __device__ __forceinline__ unsigned stage_bar_setup(unsigned long long *bar_mem)
 // BULK: every zone the launch walks has kZoneBulk (the launcher checks)
 template <int NS, int INV, int DIR, int MINB, int PART, int NT, bool BULK>
 static __global__ void __launch_bounds__(FluxBounds<MINB>::threads, FluxBounds<MINB>::blocks)
-    flux_dir_staged(DevZone z, int nchunk, int accumulate, int viscous) {
+    flux_dir_staged(DevZone z, int nchunk, int accumulate, int flags) {
   extern __shared__ __align__(16) double smem[];
   __shared__ unsigned long long bar_mem;
   const unsigned bar = stage_bar_setup(&bar_mem);
   unsigned phase = 0;
-  flux_tile_staged<NS, INV, DIR, PART, NT, BULK>(z, blockIdx.x, blockIdx.y, blockIdx.z, nchunk, accumulate, viscous,
+  flux_tile_staged<NS, INV, DIR, PART, NT, BULK>(z, blockIdx.x, blockIdx.y, blockIdx.z, nchunk, accumulate, flags,
                                                  smem, bar, phase);
 }
 
 template <int NS, int INV, int DIR, int MINB, int PART, int NT, bool BULK>
 static __global__ void __launch_bounds__(FluxBounds<MINB>::threads, FluxBounds<MINB>::blocks)
-    flux_dir_staged_table(const int4 *tiles, int n_tiles, int nchunk, int accumulate, int viscous) {
+    flux_dir_staged_table(const int4 *tiles, int n_tiles, int nchunk, int accumulate, int flags) {
   extern __shared__ __align__(16) double smem[];
   __shared__ unsigned long long bar_mem;
   const unsigned bar = stage_bar_setup(&bar_mem);
   unsigned phase = 0;
   for (int t = blockIdx.x; t < n_tiles; t += gridDim.x) {
     const int4 c = tiles[t];
-    if (!flux_tile_staged<NS, INV, DIR, PART, NT, BULK>(c_zones[c.x], c.y, c.z, c.w, nchunk, accumulate, viscous,
+    if (!flux_tile_staged<NS, INV, DIR, PART, NT, BULK>(c_zones[c.x], c.y, c.z, c.w, nchunk, accumulate, flags,
                                                         smem, bar, phase))
       return;
   }
@@ -651,9 +653,10 @@ static cudaError_t launch_flux_sb(const DevZone &z, const TileShape &t, const Fl
     if (e != cudaSuccess) return e;
   }
   const dim3 blk(32, R);
+  const int flags = (viscous ? 1 : 0) | (z.flags & kZoneHold);  // (of tables: the context's first zone, as every zone)
   if (!tab) {
     flux_dir_staged<NS, INV, DIR, MINB, PART, NT, BULK><<<flux_grid(z.mx, z.my, z.mz, DIR, R, C), blk, smem, s>>>(
-        z, C, accumulate, viscous);
+        z, C, accumulate, flags);
     return cudaGetLastError();
   }
   if (tab->n <= 0) return cudaSuccess;
@@ -664,7 +667,7 @@ static cudaError_t launch_flux_sb(const DevZone &z, const TileShape &t, const Fl
   const int slots = per_sm * sms;
   const int grid = tab->n < slots ? tab->n : slots;
   flux_dir_staged_table<NS, INV, DIR, MINB, PART, NT, BULK><<<grid, blk, smem, s>>>(tab->tiles, tab->n, C, accumulate,
-                                                                              viscous);
+                                                                              flags);
   return cudaGetLastError();
 }
 
