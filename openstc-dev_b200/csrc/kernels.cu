@@ -879,21 +879,17 @@ __device__ __forceinline__ void bc_point(const DevZone &z, const BcFace &b, int 
 template <int NS>
 __device__ __forceinline__ void interface_point(const DevZone &z, const DevZone &t, const Iface &f, int with_cv,
                                                 int n0, int n1, int n2) {
-  const int n[3] = {n0, n1, n2};
-  int idx[3], d[3], it[3];
-#pragma unroll
-  for (int a = 0; a < 3; ++a) {
-    d[a] = f.ld[a] * n[a];
-    idx[a] = f.rs[a] + d[a];
-  }
-#pragma unroll
-  for (int a = 0; a < 3; ++a) it[a] = f.ts[a] + f.tld[a] * d[f.st[a]];
-  const int g = gidx(z, idx[0], idx[1], idx[2]);
-  const int gt = gidx(t, it[0], it[1], it[2]);
+  // by selection: arrays indexed by the face's axes went to local memory
+  const int d0 = f.ld[0] * n0, d1 = f.ld[1] * n1, d2 = f.ld[2] * n2;
+  auto of = [](int a, int x, int y, int z) { return a == 0 ? x : (a == 1 ? y : z); };
+  auto partner = [&](int a) { return f.ts[a] + f.tld[a] * of(f.st[a], d0, d1, d2); };
+  const int i = f.rs[0] + d0, j = f.rs[1] + d1, k = f.rs[2] + d2;
+  const int g = gidx(z, i, j, k);
+  const int gt = gidx(t, partner(0), partner(1), partner(2));
   const int plane = f.direction > 0 ? f.rs[f.face] : f.rs[f.face] + f.ld[f.face] * (f.np[f.face] - 1);
   PointState<NS> s;
   load_point<NS>(t, gt, s);
-  if (idx[f.face] == plane) {
+  if (of(f.face, i, j, k) == plane) {
     PointState<NS> o;
     load_point<NS>(z, g, o);
 #pragma unroll
