@@ -804,9 +804,11 @@ void build_devparam(const ostc_param *p, DevParam &d) {
 //    against 267 for the 128-register plane kernel);
 //    Air with SST likewise (96 x 96 x 96: 156 / 145 / 141 against 334 / 352 / 377), but
 //    where its blocks have both odd and even rows, which the staged kernels take in a
-//    launch each: then plane kernels of 80 registers (5 blocks of 492000 cells: 112 / 145
-//    / 134 against 133 / 149 / 151 staged), or of 128 for fewer than eight waves (5
-//    blocks of 132000 cells: 29 / 45 / 45 against 45 / 58 / 58);
+//    launch each: then plane kernels, but for y and z sweeps of sixteen waves or more (13
+//    blocks of 1.9 M cells: staged 403 / 413 / 424, 80 registers 349 / 433 / 458), of 80
+//    registers (5 blocks of 492000 cells: 112 / 145 / 134 against 133 / 149 / 151 staged)
+//    or, for fewer than eight waves, of 128 (5 blocks of 132000 cells: 29 / 45 / 45
+//    against 45 / 58 / 58);
 //  - air: plane kernels of 80 registers (157 x 99 x 67: 114 / 131 / 143 against 165 /
 //    323 / 287, staged 139 / 147 / 148; Roe 147 / 173 / 182 against 220 / 444 / 393);
 //  - AWENO (no staged build, 240 registers wanted) and the rest: plane kernels of 128
@@ -837,7 +839,7 @@ void default_tiles(ostc_ctx *c) {
     };
     const size_t smem = stage_smem_bytes(c->ns, c->nt, d, viscous) + 64 * (5 + c->ns + c->nt) + 1024;
     const bool staged = !aweno && ((c->ns > 0 && !roe) || c->nt > 0) && 2 * smem <= 228 * 1024 &&
-                        !(air_sst && even && odd);
+                        !(air_sst && even && odd && (d == 0 || tiles(8, 1) < 16 * 2 * sms));
     if (!staged || air_sst) {
       const int rows = tiles(4, 1) <= 2 * sms ? 4 : (tiles(8, 1) <= sms ? 8 : 0);
       if (rows) {
