@@ -176,8 +176,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1) gemm_tc_kernel(TcGemmArgs g) {
       // four 16-byte stores, and transposed (the K-major operand of the weight gradient),
       // where a column's 32 rows are 64 contiguous bytes: neighbouring lanes exchange rows
       // so that each stores two (even lanes of column j, odd lanes of column j + 1), zeros
-      // up to the padded length. A warp whose rows all lie beyond that has none
-      if (g.act && r0 < g.ldt) {
+      // up to the padded length
+      if (g.act) {
         const bool row = r0 + lane < g.M;
         unsigned own[16];  // columns j, j + 1 of this row
 #pragma unroll
