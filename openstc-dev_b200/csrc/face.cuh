@@ -115,9 +115,9 @@ __device__ __forceinline__ double minmod(double a, double b) {
 // J. Res. Dev. 34, 1990), three operations instead of about twenty. Used where
 // plain products with r showed in a residual's error against extended precision
 // (2-norms): the density's with AUSM+, 9.4e-15 with divisions or corrected,
-// 9.8e-15 without (nine species 6.2e-15 and 7.4e-15); AWENO's 2.37e-14 with
-// divisions, 2.45e-14 without, 2.38e-14 with the velocities corrected (and p / rho
-// from the specific energy).
+// 9.8e-15 without (nine species 6.2e-15 and 7.4e-15); AWENO's, 2.3 % above that
+// with divisions without, 0.6 % with the velocities corrected and p / rho from the
+// specific energy.
 __device__ __forceinline__ double quotient(double a, double b, double r) {
   const double q = a * r;
   return fma(fma(-q, b, a), r, q);
